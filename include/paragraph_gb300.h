@@ -105,7 +105,7 @@ typedef struct pg_handle_s* pg_handle;
 /* Launch-shape choices of a handle.  None of them changes a result: every choice builds the same
  * graph bit for bit; they only move time.  Zero fields mean the library's defaults. */
 typedef struct pg_tuning {
-  uint32_t search_rows;         /* candidate rows staged per pass in the Km=32 search: 8 or 16 */
+  uint32_t search_rows;         /* candidate rows scored per pass in the Km=32 search: 8 or 16 */
   uint32_t search_warps_per_sm; /* cap on resident search warps per SM (0 = occupancy maximum) */
   uint32_t hash_factor;         /* visited-set capacity multiplier over the exact minimum: 1, 2, 4 */
   uint32_t screen_stages;       /* row-copy ring depth of the screened prune: 0 (= 2), 2, 3, 4 */

@@ -204,10 +204,12 @@ uint32_t pow2_at_least(uint32_t x) {
   return p;
 }
 
-// Visited-set capacity: at most km + reset_iter * kp*kd ids live between rebuilds; twice that
-// (a power of two) keeps the open-addressing table at most half full, so the set stays exact.
+// Visited-set capacity: at most km + reset_iter * kp*kd ids live between rebuilds; a power of two
+// of at least 1.6 times that keeps the open-addressing table at most 5/8 full, so the set stays
+// exact and probes stay short.
 uint32_t hash_slots_for(uint32_t km, uint32_t reset_iter, uint32_t batch) {
-  return pow2_at_least(2 * (km + reset_iter * batch));
+  const uint32_t live = km + reset_iter * batch;
+  return pow2_at_least(live + (live * 3 + 4) / 5);
 }
 
 int check_params(const pg_params* p, uint64_t n, uint32_t d, uint64_t q) {
@@ -396,7 +398,6 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.reset_iter = p->reset_iter;
       sa.seed_base = p->seed_base;
       sa.max_iters = p->max_search_iters;
-      sa.order = nullptr;
       sa.out = sres;
       sa.out_width = L;
       sa.evals = cnt + C_SEARCH + r;
@@ -1070,7 +1071,6 @@ int pg_search(pg_handle h, const float* d_base, uint64_t n, uint32_t d, const ui
   a.reset_iter = reset_iter;
   a.seed_base = seed_base;
   a.max_iters = max_iters;
-  a.order = nullptr;
   a.out = d_out;
   a.evals = h->d_counters;
   a.iters = h->d_counters + 1;

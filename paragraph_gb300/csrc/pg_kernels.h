@@ -62,7 +62,6 @@ struct SearchArgs {
   uint32_t graph_degree;
   uint32_t km, kp, kd, reset_iter, seed_base;
   uint32_t max_iters;
-  const uint32_t* order;  // optional query order (permutation of 0..n-1), NULL = identity
   uint32_t* out;          // n x (km + kp*kd)
   unsigned long long* evals;
   unsigned long long* iters;
@@ -76,7 +75,7 @@ struct SearchArgs {
   const float* queries;
   uint64_t nq;
   uint32_t out_width;  // ids written per query: L for link rounds, top-k for a query search
-  // launch shape (results do not depend on it): candidate rows staged per pass (8 or 16, Km = 32
+  // launch shape (results do not depend on it): candidate rows scored per pass (8 or 16, Km = 32
   // kernel) and a cap on resident search warps per SM; 0 = defaults
   uint32_t rows;
   uint32_t max_blocks_per_sm;

@@ -410,7 +410,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.rows = h->tune.search_rows;
       sa.max_blocks_per_sm = h->tune.search_warps_per_sm;
       // the queries (the base points) and their seeds are the same in every round
-      if (r == 0) PG_CUDA(pg::launch_seed_dists(sa, seeds, sms, s));
+      if (r == 0) PG_CUDA(pg::launch_seed_dists(sa, seeds, sms, h->smem_optin, s));
       sa.seed_dist = seeds;
       PG_CUDA(pg::launch_search(sa, sms, h->smem_optin, s));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[2 + 3 * r], s));

@@ -197,7 +197,8 @@ cudaError_t launch_copy16(void* dst, const void* src, uint64_t bytes, int num_sm
 // (see search_supported).
 cudaError_t launch_search(const SearchArgs& a, int num_sms, size_t smem_optin, cudaStream_t st);
 // Every query's 32 seed distances in the search's FP32 order into out (queries x 32).
-cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms, cudaStream_t st);
+cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms, size_t smem_optin,
+                              cudaStream_t st);
 bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd);
 // Screened prune for strict rounds (pg_prune_tc.cu): FP16 or BF16 candidate Gram on the tcgen05
 // tensor cores + exact re-scoring, 1 <= c <= 128, 4 <= d <= 1024, d % 4 == 0; the launch also

@@ -485,59 +485,130 @@ static cudaError_t launch_search_k(const SearchArgs& a, int num_sms, size_t smem
 
 // The distances of every query to its 32 seeds ((seed_base + s) % n_sub + offset), in the
 // search's FP32 order (Gsearcher.cuh:958-976): residue r = i mod 32 accumulates q[i]*x[i] in i
-// order, then the shuffle-down tree 16, 8, 4, 2, 1.  Lane s holds seed s's 32 residue chains in
-// registers and folds them in the tree's pairs.  The seeds of one (sub-)index are the same 32
-// rows for every query, so they stay in L1; this pass replaces the four staging passes per query
-// and round that scoring the seeds inside the search takes.  One warp per query.
-__global__ void __launch_bounds__(256) k_seed_dists(SearchArgs a, float* __restrict__ out) {
-  const uint32_t lane = lane_id();
+// order, then the shuffle-down tree 16, 8, 4, 2, 1.  Lane s holds seed s's 32 residue chains of
+// kSeedQ queries in registers and folds them in the tree's pairs.  The seeds of one (sub-)index
+// are the same 32 rows for every query: a block stages them in shared memory (row stride an odd
+// number of float4, so the 32 lanes read their rows without bank conflicts) and keeps them for
+// its whole range of queries, whose rows stream through two shared tiles filled one tile ahead.
+// Per float4 step a warp takes one shared load of seeds (four wavefronts) and kSeedQ broadcast
+// loads for 4 kSeedQ FMAs.
+constexpr int kSeedQ = 4;
+constexpr uint32_t kSeedWarps = 8;
+constexpr uint32_t kSeedTile = kSeedWarps * kSeedQ;  // queries per tile
+
+__host__ __device__ __forceinline__ uint32_t seed_stride4(uint32_t d) { return (d / 4) | 1u; }
+
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+
+__global__ void __launch_bounds__(32 * kSeedWarps) k_seed_dists(SearchArgs a,
+                                                                float* __restrict__ out) {
+  extern __shared__ __align__(16) float4 seeds4[];
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   const uint64_t nq = a.queries ? a.nq : a.n;
-  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
-  const uint32_t d = a.d;
-  for (uint64_t qid = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
-       qid < nq; qid += nw) {
-    uint64_t soff = 0, sn = a.n;
+  const uint32_t d = a.d, d4 = d / 4, stride = seed_stride4(d);
+  float4* tiles = seeds4 + 32u * stride;  // two tiles of kSeedTile rows
+  const float4* rows = reinterpret_cast<const float4*>(a.queries ? a.queries : a.base);
+  const uint64_t tiles_all = (nq + kSeedTile - 1) / kSeedTile;
+  const uint64_t per = (tiles_all + gridDim.x - 1) / gridDim.x * kSeedTile;
+  const uint64_t end = min(nq, per * (blockIdx.x + 1));
+  for (uint64_t q0 = per * blockIdx.x; q0 < end;) {
+    uint64_t soff = 0, sn = a.n, stop = end;  // this block's queries of one sub-index
     if (a.seg_count) {
-      const uint32_t sg = segment_of(a.seg_off, a.seg_count, qid);
+      const uint32_t sg = segment_of(a.seg_off, a.seg_count, q0);
       soff = a.seg_off[sg];
       sn = a.seg_off[sg + 1] - soff;
+      stop = min(end, soff + sn);
     }
-    const uint64_t node = (a.seed_base + static_cast<uint64_t>(lane)) % sn + soff;
-    const float4* q4 =
-        reinterpret_cast<const float4*>((a.queries ? a.queries : a.base) + qid * d);
-    const float4* x4 = reinterpret_cast<const float4*>(a.base + node * d);
-    float s[32];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < 32u * d4; i += blockDim.x) {
+      const uint32_t r = i / d4, c = i - r * d4;
+      const uint64_t node = (a.seed_base + static_cast<uint64_t>(r)) % sn + soff;
+      seeds4[r * stride + c] = __ldg(reinterpret_cast<const float4*>(a.base + node * d) + c);
+    }
+    auto fill = [&](uint64_t t0, uint32_t buf) {  // a tile is one contiguous range
+      if (t0 < stop) {
+        const uint32_t words = static_cast<uint32_t>(min(stop - t0, uint64_t(kSeedTile))) * d4;
+        float4* dst = tiles + buf * kSeedTile * d4;
+        const float4* src = rows + t0 * d4;
+        for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) cp16(dst + i, src + i);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    uint32_t buf = 0;
+    fill(q0, 0);
+    const float4* x4 = seeds4 + lane * stride;
+    for (uint64_t t0 = q0; t0 < stop; t0 += kSeedTile, buf ^= 1u) {
+      fill(t0 + kSeedTile, buf ^ 1u);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      const float4* q4 = tiles + (buf * kSeedTile + warp * kSeedQ) * d4;
+      const uint64_t qb = t0 + warp * kSeedQ;
+      if (qb < stop) {
+        float s[kSeedQ][32];  // rows past the end hold an earlier tile's or no data: not written
 #pragma unroll
-    for (int r = 0; r < 32; r++) s[r] = 0.f;
-    for (uint32_t b = 0; b < d; b += 32) {
+        for (int t = 0; t < kSeedQ; t++)
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        if (b + 4u * j < d) {
-          const float4 q = __ldg(q4 + (b >> 2) + j);
-          const float4 x = __ldg(x4 + (b >> 2) + j);
-          s[4 * j] = fmaf(q.x, x.x, s[4 * j]);
-          s[4 * j + 1] = fmaf(q.y, x.y, s[4 * j + 1]);
-          s[4 * j + 2] = fmaf(q.z, x.z, s[4 * j + 2]);
-          s[4 * j + 3] = fmaf(q.w, x.w, s[4 * j + 3]);
+          for (int r = 0; r < 32; r++) s[t][r] = 0.f;
+        auto step = [&](uint32_t b, uint32_t j) {
+          const float4 x = x4[b + j];
+#pragma unroll
+          for (int t = 0; t < kSeedQ; t++) {
+            const float4 q = q4[t * d4 + b + j];
+            s[t][4 * j] = fmaf(q.x, x.x, s[t][4 * j]);
+            s[t][4 * j + 1] = fmaf(q.y, x.y, s[t][4 * j + 1]);
+            s[t][4 * j + 2] = fmaf(q.z, x.z, s[t][4 * j + 2]);
+            s[t][4 * j + 3] = fmaf(q.w, x.w, s[t][4 * j + 3]);
+          }
+        };
+        uint32_t b = 0;
+#pragma unroll 1
+        for (; b + 8 <= d4; b += 8) {
+#pragma unroll
+          for (uint32_t j = 0; j < 8; j++) step(b, j);
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 8; j++)
+          if (b + j < d4) step(b, j);
+#pragma unroll
+        for (int t = 0; t < kSeedQ; t++) {
+#pragma unroll
+          for (int w = 16; w >= 1; w >>= 1)
+#pragma unroll
+            for (int r = 0; r < w; r++) s[t][r] = s[t][r] + s[t][r + w];
+          if (qb + t < stop) out[(qb + t) * 32u + lane] = -s[t][0];
         }
       }
+      __syncthreads();  // the tile is overwritten two fills later
     }
-#pragma unroll
-    for (int w = 16; w >= 1; w >>= 1)
-#pragma unroll
-      for (int r = 0; r < w; r++) s[r] = s[r] + s[r + w];
-    out[qid * 32u + lane] = -s[0];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    q0 = stop;
   }
 }
 
-cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms, cudaStream_t st) {
+cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms,
+                              size_t smem_optin, cudaStream_t st) {
   if (a.d == 0 || (a.d % 4) != 0 || !out) return cudaErrorInvalidValue;
   const uint64_t nq = a.queries ? a.nq : a.n;
   if (nq == 0) return cudaSuccess;
-  uint64_t blocks = (nq + 7) / 8;
-  const uint64_t cap = static_cast<uint64_t>(num_sms) * 8;
+  const size_t smem = 32 * static_cast<size_t>(seed_stride4(a.d)) * 16 +
+                      2 * kSeedTile * static_cast<size_t>(a.d) * 4;
+  if (smem > smem_optin) return cudaErrorInvalidValue;
+  auto kern = k_seed_dists;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * kSeedWarps, smem);
+  if (e != cudaSuccess) return e;
+  uint64_t blocks = (nq + kSeedTile - 1) / kSeedTile;
+  const uint64_t cap = static_cast<uint64_t>(num_sms) * (per_sm < 1 ? 1 : per_sm);
   if (blocks > cap) blocks = cap;
-  k_seed_dists<<<static_cast<unsigned>(blocks), 256, 0, st>>>(a, out);
+  kern<<<static_cast<unsigned>(blocks), 32 * kSeedWarps, smem, st>>>(a, out);
   return cudaGetLastError();
 }
 

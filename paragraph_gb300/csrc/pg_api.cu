@@ -70,11 +70,11 @@ size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 struct Layout {
   size_t winner, pruned, pruned_num, indeg, offs, tile_sums, cursor, edges, rev, rev_num, sres,
-      proj, graph, segs, norms, seeds, total;
+      proj, graph, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place, total;
 };
 
-Layout make_layout(uint64_t n, uint32_t pmax, uint32_t rmax, uint32_t L, uint32_t proj_deg,
-                   uint32_t degree, uint32_t seg_count = 0) {
+Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_t L,
+                   uint32_t proj_deg, uint32_t degree, uint32_t nkeys, uint32_t seg_count = 0) {
   Layout l{};
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -98,6 +98,16 @@ Layout make_layout(uint64_t n, uint32_t pmax, uint32_t rmax, uint32_t L, uint32_
   l.segs = take(2 * (static_cast<size_t>(seg_count) + 1) * 8);
   l.norms = take(n * 8);  // screened prune: per-point norm bounds
   l.seeds = take(n * 32 * 4);  // link-round searches: every query's 32 seed distances
+  if (nkeys) {  // relocated build: the sorted copy of the base, seed distances and graphs by place
+    l.rbase = take(n * d * 4);
+    l.rseeds = take(n * 32 * 4);
+    l.rproj = take(n * proj_deg * 4);
+    l.rgraph = take(n * degree * 4);
+    l.keys = take(n * 4);
+    l.bins = take(nkeys * 4);
+    l.order = take(n * 4);
+    l.place = take(n * 4);
+  }
   l.total = o;
   return l;
 }
@@ -127,6 +137,7 @@ struct pg_handle_s {
   size_t smem_optin = 0;
   char* ws = nullptr;
   size_t ws_bytes = 0;
+  size_t reloc_limit = ~static_cast<size_t>(0);  // a relocated build's workspace did not fit
   char* inbuf = nullptr;  // device copies of host inputs (pg_build_host)
   size_t in_bytes = 0;
   uint32_t* d_status = nullptr;
@@ -286,8 +297,22 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   const uint32_t L = p->km + p->kp * p->kd;
   const uint32_t pmax = std::max(p->proj_pruned, p->degree);
   const uint32_t rmax = std::max(p->proj_reverse, p->link_reverse);
-  Layout lay = make_layout(n, pmax, rmax, L, p->proj_degree, p->degree, seg_count);
+  uint32_t nkeys = p->link_rounds ? pg::reloc_keys(n, d, seg_count) : 0;
+  auto shape = [&]() {
+    return make_layout(n, d, pmax, rmax, L, p->proj_degree, p->degree, nkeys, seg_count);
+  };
+  Layout lay = shape();
+  if (nkeys && lay.total >= h->reloc_limit) {
+    nkeys = 0;
+    lay = shape();
+  }
   int rc = ensure_ws(h, lay.total);
+  if (rc == PG_ENOMEM && nkeys) {  // no room for the copy: build on the caller's rows
+    h->reloc_limit = lay.total;
+    nkeys = 0;
+    lay = shape();
+    rc = ensure_ws(h, lay.total);
+  }
   if (rc) return rc;
   char* w = h->ws;
   uint32_t* winner = reinterpret_cast<uint32_t*>(w + lay.winner);
@@ -301,9 +326,13 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   uint32_t* rev = reinterpret_cast<uint32_t*>(w + lay.rev);
   uint32_t* rnum = reinterpret_cast<uint32_t*>(w + lay.rev_num);
   uint32_t* sres = reinterpret_cast<uint32_t*>(w + lay.sres);
-  uint32_t* proj = proj_out ? proj_out : reinterpret_cast<uint32_t*>(w + lay.proj);
+  uint32_t* proj = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rproj)
+                   : proj_out ? proj_out : reinterpret_cast<uint32_t*>(w + lay.proj);
+  uint32_t* link = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rgraph) : graph_out;
   float2* norms = reinterpret_cast<float2*>(w + lay.norms);
   float* seeds = reinterpret_cast<float*>(w + lay.seeds);
+  uint32_t* order = nkeys ? reinterpret_cast<uint32_t*>(w + lay.order) : nullptr;
+  uint32_t* place = nkeys ? reinterpret_cast<uint32_t*>(w + lay.place) : nullptr;
   const bool screened = p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1);
   unsigned long long* cnt = h->d_counters;
   const int sms = h->num_sms;
@@ -334,12 +363,39 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     PG_CUDA(cudaMemsetAsync(h->d_work, 0, 8 * sizeof(uint32_t), s));
     if (stage_events) PG_CUDA(cudaEventRecord(h->ev[0], s));
 
+    // the link rounds' seed distances (every point is a query, the same in every round), and the
+    // relocated copy that the stages below work on
+    const float* rows = base;
+    const float* seed_dist = seeds;
+    if (p->link_rounds) {
+      pg::SearchArgs qa{};
+      qa.base = base;
+      qa.n = n;
+      qa.d = d;
+      qa.seed_base = p->seed_base;
+      qa.seg_off = d_seg;
+      qa.seg_count = seg_count;
+      uint32_t* keys = nkeys ? reinterpret_cast<uint32_t*>(w + lay.keys) : nullptr;
+      uint32_t* bins = nkeys ? reinterpret_cast<uint32_t*>(w + lay.bins) : nullptr;
+      if (nkeys) PG_CUDA(cudaMemsetAsync(bins, 0, nkeys * 4, s));
+      PG_CUDA(pg::launch_seed_dists(qa, seeds, keys, bins, sms, h->smem_optin, s));
+      if (nkeys) {
+        float* rbase = reinterpret_cast<float*>(w + lay.rbase);
+        float* rseeds = reinterpret_cast<float*>(w + lay.rseeds);
+        PG_CUDA(pg::launch_reloc_order(keys, n, bins, nkeys, order, place, sms, s));
+        PG_CUDA(pg::launch_reloc_rows(base, n, d, seeds, order, rbase, rseeds, sms, s));
+        rows = rbase;
+        seed_dist = rseeds;
+      }
+    }
+    if (stage_events) PG_CUDA(cudaEventRecord(h->ev[15], s));
+
     // K0 projection winners; K1+K2 phase-1 prune (rows read from gt through the winner)
     PG_CUDA(pg::launch_match_winner(gt, q, p->gt_k, n, winner, h->d_status, sms, s, d_seg, d_qseg,
-                                    seg_count));
+                                    seg_count, place));
     PG_CUDA(cudaMemsetAsync(indeg, 0, n * 4, s));
     pg::PruneArgs pa{};
-    pa.base = base;
+    pa.base = rows;
     pa.n = n;
     pa.d = d;
     pa.graph = nullptr;
@@ -358,13 +414,14 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     pa.seg_off = d_seg;
     pa.qseg_off = d_qseg;
     pa.seg_count = seg_count;
+    pa.place = place;
     PG_CUDA(pg::launch_prune_reverse(pa, true, sms, s));
     PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->proj_pruned, n, indeg, offs, tsum, cursor, edges,
-                                   sms, s));
-    PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->proj_reverse, rev, rnum, sms, s));
+                                   sms, s, 0, order));
+    PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->proj_reverse, rev, rnum, sms, s, place));
     // K3 phase-1 merge -> projection graph
     pg::MergeArgs ma{};
-    ma.base = base;
+    ma.base = rows;
     ma.n = n;
     ma.d = d;
     ma.pruned = pruned;
@@ -387,7 +444,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
                             std::max(1u, h->tune.hash_factor);
     for (uint32_t r = 0; r < p->link_rounds; r++) {
       pg::SearchArgs sa{};
-      sa.base = base;
+      sa.base = rows;
       sa.n = n;
       sa.d = d;
       sa.graph = g;
@@ -398,6 +455,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.reset_iter = p->reset_iter;
       sa.seed_base = p->seed_base;
       sa.max_iters = p->max_search_iters;
+      sa.place = place;
       sa.out = sres;
       sa.out_width = L;
       sa.evals = cnt + C_SEARCH + r;
@@ -409,14 +467,12 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.seg_count = seg_count;
       sa.rows = h->tune.search_rows;
       sa.max_blocks_per_sm = h->tune.search_warps_per_sm;
-      // the queries (the base points) and their seeds are the same in every round
-      if (r == 0) PG_CUDA(pg::launch_seed_dists(sa, seeds, sms, h->smem_optin, s));
-      sa.seed_dist = seeds;
+      sa.seed_dist = seed_dist;
       PG_CUDA(pg::launch_search(sa, sms, h->smem_optin, s));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[2 + 3 * r], s));
       PG_CUDA(cudaMemsetAsync(indeg, 0, n * 4, s));
       pg::PruneArgs pr{};
-      pr.base = base;
+      pr.base = rows;
       pr.n = n;
       pr.d = d;
       pr.graph = sres;
@@ -435,16 +491,16 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       pr.norms = norms;
       if (screened) {
         if (r == 0)
-          PG_CUDA(pg::launch_screen_norms(base, n, d, pr.screen_half, norms, sms, s));
+          PG_CUDA(pg::launch_screen_norms(rows, n, d, pr.screen_half, norms, sms, s));
         PG_CUDA(pg::launch_prune_screen(pr, sms, h->smem_optin, s));
       } else
         PG_CUDA(pg::launch_prune_reverse(pr, false, sms, s));
       PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->degree, n, indeg, offs, tsum, cursor, edges,
-                                     sms, s));
-      PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->link_reverse, rev, rnum, sms, s));
+                                     sms, s, 0, order));
+      PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->link_reverse, rev, rnum, sms, s, place));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[3 + 3 * r], s));
       pg::MergeArgs mr{};
-      mr.base = base;
+      mr.base = rows;
       mr.n = n;
       mr.d = d;
       mr.pruned = pruned;
@@ -455,12 +511,12 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       mr.r = p->link_reverse;
       mr.degree = p->degree;
       mr.strict = 1;
-      mr.out = graph_out;
+      mr.out = link;
       mr.evals = cnt + C_MERGE + r;
       mr.status = h->d_status;
       PG_CUDA(pg::launch_merge_prune(mr, sms, s));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[4 + 3 * r], s));
-      g = graph_out;
+      g = link;
       gdeg = p->degree;
     }
     if (p->link_rounds == 0 && graph_out) {
@@ -470,11 +526,17 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
                                 std::min(p->degree, p->proj_degree) * 4, n,
                                 cudaMemcpyDeviceToDevice, s));
     }
-    if (seg_count) {  // global ids -> ids local to each sub-index
+    if (nkeys) {  // places -> the caller's ids and rows
+      PG_CUDA(pg::launch_restore(link, n, p->degree, order, d_seg, seg_count, graph_out, sms, s));
+      if (proj_out)
+        PG_CUDA(pg::launch_restore(proj, n, p->proj_degree, order, d_seg, seg_count, proj_out, sms,
+                                   s));
+    } else if (seg_count) {  // global ids -> ids local to each sub-index
       if (graph_out && p->link_rounds > 0)
         PG_CUDA(pg::launch_localize(graph_out, n, p->degree, d_seg, seg_count, sms, s));
       PG_CUDA(pg::launch_localize(proj, n, p->proj_degree, d_seg, seg_count, sms, s));
     }
+    if (stage_events) PG_CUDA(cudaEventRecord(h->ev[14], s));
     PG_CUDA(cudaMemcpyAsync(h->h_status, h->d_status, 4, cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaMemcpyAsync(h->h_counters, cnt, C_COUNT * 8, cudaMemcpyDeviceToHost, s));
     return PG_OK;
@@ -538,7 +600,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     if (use_graph) {  // one replay, timed as a whole
       PG_CUDA(cudaEventElapsedTime(&st->ms_total, h->ev[14], h->ev[15]));
     } else {
-      PG_CUDA(cudaEventElapsedTime(&st->ms_proj, h->ev[0], h->ev[1]));
+      PG_CUDA(cudaEventElapsedTime(&st->ms_proj, h->ev[15], h->ev[1]));
       cudaEvent_t prev = h->ev[1];
       for (uint32_t r = 0; r < p->link_rounds; r++) {
         PG_CUDA(cudaEventElapsedTime(&st->ms_search[r], prev, h->ev[2 + 3 * r]));
@@ -546,7 +608,12 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
         PG_CUDA(cudaEventElapsedTime(&st->ms_merge[r], h->ev[3 + 3 * r], h->ev[4 + 3 * r]));
         prev = h->ev[4 + 3 * r];
       }
-      PG_CUDA(cudaEventElapsedTime(&st->ms_total, h->ev[0], prev));
+      if (p->link_rounds) {  // round 1's search time holds the pre-passes it needs
+        float ms = 0.0f;
+        PG_CUDA(cudaEventElapsedTime(&ms, h->ev[0], h->ev[15]));
+        st->ms_search[0] += ms;
+      }
+      PG_CUDA(cudaEventElapsedTime(&st->ms_total, h->ev[0], h->ev[14]));
     }
   }
   return PG_OK;
@@ -808,8 +875,9 @@ int pg_workspace_bytes(const pg_params* p, uint64_t n, uint32_t d, uint64_t q, u
   if (rc) return rc;
   if (!bytes) return fail(PG_EINVAL, "bytes is NULL");
   const uint32_t L = p->km + p->kp * p->kd;
-  Layout l = make_layout(n, std::max(p->proj_pruned, p->degree),
-                         std::max(p->proj_reverse, p->link_reverse), L, p->proj_degree, p->degree);
+  Layout l = make_layout(n, d, std::max(p->proj_pruned, p->degree),
+                         std::max(p->proj_reverse, p->link_reverse), L, p->proj_degree, p->degree,
+                         p->link_rounds ? pg::reloc_keys(n, d, 0) : 0);
   *bytes = l.total;
   return PG_OK;
 }

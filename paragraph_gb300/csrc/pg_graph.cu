@@ -32,7 +32,8 @@ __device__ __forceinline__ uint32_t winner_query(uint32_t key) {
 __global__ void k_match_winner(const uint32_t* __restrict__ gt, uint64_t q, uint32_t gt_k,
                                uint64_t n, uint32_t* __restrict__ winner, uint32_t* status,
                                const uint64_t* __restrict__ seg_off,
-                               const uint64_t* __restrict__ qseg_off, uint32_t seg_count) {
+                               const uint64_t* __restrict__ qseg_off, uint32_t seg_count,
+                               const uint32_t* __restrict__ place) {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t qi = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; qi < q;
        qi += stride) {
@@ -48,7 +49,7 @@ __global__ void k_match_winner(const uint32_t* __restrict__ gt, uint64_t q, uint
       raise_error(status, kErrBadId);
       continue;
     }
-    const uint64_t b = bl + off;
+    const uint64_t b = place ? place[bl + off] : bl + off;
     const bool real = gt[qi * gt_k + 1] != kTomb;
     atomicMin(winner + b, winner_key(static_cast<uint32_t>(qi), real));
   }
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(256) k_prune_reverse(PruneArgs a) {
               x = kTomb;
             } else {
               x = static_cast<uint32_t>(x + goff);
+              if (a.place) x = a.place[x];
             }
           }
         } else {
@@ -469,15 +471,17 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
 __global__ void k_scatter_reverse(const uint32_t* __restrict__ pruned,
                                   const uint32_t* __restrict__ pruned_num, uint32_t p_len,
                                   uint64_t rows, const uint32_t* __restrict__ offs,
-                                  uint32_t* __restrict__ cursor, uint32_t* __restrict__ edges) {
+                                  uint32_t* __restrict__ cursor, uint32_t* __restrict__ edges,
+                                  const uint32_t* __restrict__ order) {
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t b = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; b < rows;
        b += stride) {
     const uint32_t cnt = pruned_num[b];
+    const uint32_t src = order ? order[b] : static_cast<uint32_t>(b);
     for (uint32_t t = 0; t < cnt; t++) {
       const uint32_t dst = pruned[b * p_len + t];
       const uint32_t pos = atomicAdd(cursor + dst, 1u);
-      edges[offs[dst] + pos] = static_cast<uint32_t>(b);
+      edges[offs[dst] + pos] = src;
     }
   }
 }
@@ -489,7 +493,8 @@ __global__ void __launch_bounds__(256) k_reverse_lists(const uint32_t* __restric
                                                        const uint32_t* __restrict__ edges,
                                                        uint64_t n, uint32_t r,
                                                        uint32_t* __restrict__ rev,
-                                                       uint32_t* __restrict__ rev_num) {
+                                                       uint32_t* __restrict__ rev_num,
+                                                       const uint32_t* __restrict__ place) {
   const uint32_t lane = lane_id();
   const uint64_t nwarps = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
   for (uint64_t p = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -527,7 +532,7 @@ __global__ void __launch_bounds__(256) k_reverse_lists(const uint32_t* __restric
 #pragma unroll
     for (int s = 0; s < 4; s++) {
       const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
-      if (i < cnt) rev[p * r + i] = best[s];
+      if (i < cnt) rev[p * r + i] = place ? place[best[s]] : best[s];
     }
     if (lane == 0) rev_num[p] = cnt;
   }
@@ -663,11 +668,12 @@ static int grid_for(uint64_t items, int per_block, int num_sms, int max_per_sm) 
 cudaError_t launch_match_winner(const uint32_t* gt, uint64_t q, uint32_t gt_k, uint64_t n,
                                 uint32_t* winner, uint32_t* status, int num_sms, cudaStream_t st,
                                 const uint64_t* seg_off, const uint64_t* qseg_off,
-                                uint32_t seg_count) {
+                                uint32_t seg_count, const uint32_t* place) {
   cudaError_t e = cudaMemsetAsync(winner, 0xFF, n * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   k_match_winner<<<grid_for(q, 256, num_sms, 8), 256, 0, st>>>(gt, q, gt_k, n, winner, status,
-                                                               seg_off, qseg_off, seg_count);
+                                                               seg_off, qseg_off, seg_count,
+                                                               place);
   return cudaGetLastError();
 }
 
@@ -684,6 +690,31 @@ __global__ void k_localize(uint32_t* __restrict__ rows, uint64_t n, uint32_t deg
 cudaError_t launch_localize(uint32_t* rows, uint64_t n, uint32_t deg, const uint64_t* seg_off,
                             uint32_t seg_count, int num_sms, cudaStream_t st) {
   k_localize<<<grid_for(n * deg, 256, num_sms, 8), 256, 0, st>>>(rows, n, deg, seg_off, seg_count);
+  return cudaGetLastError();
+}
+
+// One thread per output word: a row's words are consecutive threads, so both sides move whole rows.
+__global__ void k_restore(const uint32_t* __restrict__ rows, uint64_t n, uint32_t deg,
+                          const uint32_t* __restrict__ order, const uint64_t* __restrict__ seg_off,
+                          uint32_t seg_count, uint32_t* __restrict__ out) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n * deg;
+       i += stride) {
+    const uint64_t r = i / deg;
+    uint32_t v = rows[i];
+    if (v != kTomb) {
+      v = order[v];
+      if (seg_count) v = static_cast<uint32_t>(v - seg_off[segment_of(seg_off, seg_count, r)]);
+    }
+    out[static_cast<uint64_t>(order[r]) * deg + (i - r * deg)] = v;
+  }
+}
+
+cudaError_t launch_restore(const uint32_t* rows, uint64_t n, uint32_t deg, const uint32_t* order,
+                           const uint64_t* seg_off, uint32_t seg_count, uint32_t* out, int num_sms,
+                           cudaStream_t st) {
+  k_restore<<<grid_for(n * deg, 256, num_sms, 8), 256, 0, st>>>(rows, n, deg, order, seg_off,
+                                                                seg_count, out);
   return cudaGetLastError();
 }
 
@@ -729,7 +760,8 @@ cudaError_t launch_prune_reverse(const PruneArgs& a, bool phase1, int num_sms, c
 cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_num, uint32_t p_len,
                                uint64_t n, const uint32_t* indeg, uint32_t* offs,
                                uint32_t* tile_sums, uint32_t* cursor, uint32_t* edges,
-                               int num_sms, cudaStream_t st, uint64_t rows) {
+                               int num_sms, cudaStream_t st, uint64_t rows,
+                               const uint32_t* order) {
   if (rows == 0) rows = n;
   const uint32_t tiles = static_cast<uint32_t>((n + kScanTile - 1) / kScanTile);
   k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(indeg, n, tile_sums);
@@ -738,14 +770,16 @@ cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_nu
   cudaError_t e = cudaMemsetAsync(cursor, 0, n * sizeof(uint32_t), st);
   if (e != cudaSuccess) return e;
   k_scatter_reverse<<<grid_for(rows, 256, num_sms, 8), 256, 0, st>>>(pruned, pruned_num, p_len,
-                                                                      rows, offs, cursor, edges);
+                                                                      rows, offs, cursor, edges,
+                                                                      order);
   return cudaGetLastError();
 }
 
 cudaError_t launch_reverse_lists(const uint32_t* offs, const uint32_t* edges, uint64_t n,
                                  uint32_t r, uint32_t* rev, uint32_t* rev_num, int num_sms,
-                                 cudaStream_t st) {
-  k_reverse_lists<<<grid_for(n, 8, num_sms, 8), 256, 0, st>>>(offs, edges, n, r, rev, rev_num);
+                                 cudaStream_t st, const uint32_t* place) {
+  k_reverse_lists<<<grid_for(n, 8, num_sms, 8), 256, 0, st>>>(offs, edges, n, r, rev, rev_num,
+                                                              place);
   return cudaGetLastError();
 }
 

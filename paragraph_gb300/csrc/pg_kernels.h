@@ -28,6 +28,8 @@ struct PruneArgs {
   const uint64_t* seg_off;
   const uint64_t* qseg_off;
   uint32_t seg_count;
+  // relocated builds: place of every original id (phase 1 reads original ids from gt), else NULL
+  const uint32_t* place;
   // screened kernel: depth of its row-copy ring (0 = default, else 2..4); results do not
   // depend on it
   uint32_t stages;
@@ -82,6 +84,7 @@ struct SearchArgs {
   // optional (n or nq) x 32: each query's distances to its 32 seeds from launch_seed_dists (the
   // same values the search would compute); NULL = the search scores the seeds itself
   const float* seed_dist;
+  const uint32_t* place;  // relocated builds: place of every original id (the seeds), else NULL
 };
 
 // CPU RoarGraph path on the GPU (tests/test_t2iend.cu:365-613), pg_roar.cu.
@@ -169,10 +172,16 @@ int screen_scores(const float* a, uint64_t na, const float* b, uint64_t nb, uint
 cudaError_t launch_match_winner(const uint32_t* gt, uint64_t q, uint32_t gt_k, uint64_t n,
                                 uint32_t* winner, uint32_t* status, int num_sms, cudaStream_t st,
                                 const uint64_t* seg_off = nullptr,
-                                const uint64_t* qseg_off = nullptr, uint32_t seg_count = 0);
+                                const uint64_t* qseg_off = nullptr, uint32_t seg_count = 0,
+                                const uint32_t* place = nullptr);
 // Rewrites global ids of a batched build's rows (n x deg) to ids local to each row's sub-index.
 cudaError_t launch_localize(uint32_t* rows, uint64_t n, uint32_t deg, const uint64_t* seg_off,
                             uint32_t seg_count, int num_sms, cudaStream_t st);
+// A relocated build's rows (n x deg, by place, holding places) to the caller's: row order[i] of
+// out = row i of rows with every place x replaced by order[x], local to its sub-index.
+cudaError_t launch_restore(const uint32_t* rows, uint64_t n, uint32_t deg, const uint32_t* order,
+                           const uint64_t* seg_off, uint32_t seg_count, uint32_t* out, int num_sms,
+                           cudaStream_t st);
 cudaError_t launch_match_rows(const uint32_t* gt, uint32_t gt_k, uint64_t n,
                               const uint32_t* winner, uint32_t* out, int num_sms,
                               cudaStream_t st);
@@ -184,10 +193,13 @@ cudaError_t launch_prune_reverse(const PruneArgs& a, bool phase1, int num_sms, c
 cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_num, uint32_t p_len,
                                uint64_t n, const uint32_t* indeg, uint32_t* offs,
                                uint32_t* tile_sums, uint32_t* cursor, uint32_t* edges,
-                               int num_sms, cudaStream_t st, uint64_t rows = 0);
+                               int num_sms, cudaStream_t st, uint64_t rows = 0,
+                               const uint32_t* order = nullptr);
+// With order / place (relocated builds) the edges hold original ids, which decide which sources a
+// list keeps and their sequence, and the lists hold places.
 cudaError_t launch_reverse_lists(const uint32_t* offs, const uint32_t* edges, uint64_t n,
                                  uint32_t r, uint32_t* rev, uint32_t* rev_num, int num_sms,
-                                 cudaStream_t st);
+                                 cudaStream_t st, const uint32_t* place = nullptr);
 cudaError_t launch_merge_prune(const MergeArgs& a, int num_sms, cudaStream_t st);
 // bytes (a multiple of 16, both pointers 16-byte aligned) from src to dst by a kernel: used with
 // pinned host memory mapped into the device address space (cudaHostGetDevicePointer).
@@ -196,9 +208,22 @@ cudaError_t launch_copy16(void* dst, const void* src, uint64_t bytes, int num_sm
 // Returns cudaErrorInvalidValue for parameter combinations the search kernel was not built for
 // (see search_supported).
 cudaError_t launch_search(const SearchArgs& a, int num_sms, size_t smem_optin, cudaStream_t st);
-// Every query's 32 seed distances in the search's FP32 order into out (queries x 32).
-cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms, size_t smem_optin,
-                              cudaStream_t st);
+// Every query's 32 seed distances in the search's FP32 order into out (queries x 32).  With keys,
+// also each query's locality key (its sub-index, nearest and second nearest seed: one of
+// reloc_keys values), counted into bins (zeroed before the launch).
+cudaError_t launch_seed_dists(const SearchArgs& a, float* out, uint32_t* keys, uint32_t* bins,
+                              int num_sms, size_t smem_optin, cudaStream_t st);
+// Relocation: the build works on a copy of the base sorted by locality key.  reloc_keys is the
+// number of keys, 0 when a build of this size runs on the caller's rows.
+uint32_t reloc_keys(uint64_t n, uint32_t d, uint32_t seg_count);
+// order = the ids sorted by key (any order inside a key) and its inverse; bins: the keys' counts,
+// used up.
+cudaError_t launch_reloc_order(const uint32_t* keys, uint64_t n, uint32_t* bins, uint32_t nkeys,
+                               uint32_t* order, uint32_t* place, int num_sms, cudaStream_t st);
+// Row i of out_base / out_seeds = row order[i] of base (n x d) / seeds (n x 32).
+cudaError_t launch_reloc_rows(const float* base, uint64_t n, uint32_t d, const float* seeds,
+                              const uint32_t* order, float* out_base, float* out_seeds,
+                              int num_sms, cudaStream_t st);
 bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd);
 // Screened prune for strict rounds (pg_prune_tc.cu): FP16 or BF16 candidate Gram on the tcgen05
 // tensor cores + exact re-scoring, 1 <= c <= 128, 4 <= d <= 1024, d % 4 == 0; the launch also

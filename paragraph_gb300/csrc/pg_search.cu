@@ -285,6 +285,7 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
         sn = a.seg_off[sg + 1] - soff;
       }
       cand_id = static_cast<uint32_t>((a.seed_base + static_cast<uint64_t>(lane)) % sn + soff);
+      if (a.place) cand_id = a.place[cand_id];
       // scored for every query at once by k_seed_dists, or here
       const float dist = a.seed_dist ? a.seed_dist[static_cast<uint64_t>(qid) * 32u + lane]
                                      : score_new<KSTEPS, ROWS>(a, q, cand_id, true, list);
@@ -505,8 +506,12 @@ __device__ __forceinline__ void cp16(void* dst, const void* src) {
                : "memory");
 }
 
+template <bool KEYS>
 __global__ void __launch_bounds__(32 * kSeedWarps) k_seed_dists(SearchArgs a,
-                                                                float* __restrict__ out) {
+                                                                float* __restrict__ out,
+                                                                uint32_t* __restrict__ keys,
+                                                                uint32_t* __restrict__ bins,
+                                                                uint32_t seg_keys) {
   extern __shared__ __align__(16) float4 seeds4[];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   const uint64_t nq = a.queries ? a.nq : a.n;
@@ -518,8 +523,9 @@ __global__ void __launch_bounds__(32 * kSeedWarps) k_seed_dists(SearchArgs a,
   const uint64_t end = min(nq, per * (blockIdx.x + 1));
   for (uint64_t q0 = per * blockIdx.x; q0 < end;) {
     uint64_t soff = 0, sn = a.n, stop = end;  // this block's queries of one sub-index
+    uint32_t sg = 0;
     if (a.seg_count) {
-      const uint32_t sg = segment_of(a.seg_off, a.seg_count, q0);
+      sg = segment_of(a.seg_off, a.seg_count, q0);
       soff = a.seg_off[sg];
       sn = a.seg_off[sg + 1] - soff;
       stop = min(end, soff + sn);
@@ -580,7 +586,22 @@ __global__ void __launch_bounds__(32 * kSeedWarps) k_seed_dists(SearchArgs a,
           for (int w = 16; w >= 1; w >>= 1)
 #pragma unroll
             for (int r = 0; r < w; r++) s[t][r] = s[t][r] + s[t][r + w];
-          if (qb + t < stop) out[(qb + t) * 32u + lane] = -s[t][0];
+          if (qb + t >= stop) continue;
+          const float dist = -s[t][0];
+          out[(qb + t) * 32u + lane] = dist;
+          if (KEYS) {  // nearest and second nearest seed
+            const uint32_t k = order_key(dist);
+            const uint32_t first = __reduce_min_sync(kFull, k);
+            const uint32_t l1 = __ffs(static_cast<int>(__ballot_sync(kFull, k == first))) - 1;
+            const uint32_t k2 = lane == l1 ? 0xFFFFFFFFu : k;
+            const uint32_t second = __reduce_min_sync(kFull, k2);
+            const uint32_t l2 = __ffs(static_cast<int>(__ballot_sync(kFull, k2 == second))) - 1;
+            if (lane == 0) {
+              const uint32_t key = sg * seg_keys + (seg_keys == 32 ? l1 : l1 * 32u + l2);
+              keys[qb + t] = key;
+              atomicAdd(bins + key, 1u);
+            }
+          }
         }
       }
       __syncthreads();  // the tile is overwritten two fills later
@@ -590,15 +611,19 @@ __global__ void __launch_bounds__(32 * kSeedWarps) k_seed_dists(SearchArgs a,
   }
 }
 
-cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms,
-                              size_t smem_optin, cudaStream_t st) {
+// Keys per sub-index: nearest and second nearest seed, or the nearest alone when many sub-indexes
+// would make the table of counts large.
+static uint32_t keys_per_segment(uint32_t seg_count) { return seg_count <= 64 ? 1024u : 32u; }
+
+cudaError_t launch_seed_dists(const SearchArgs& a, float* out, uint32_t* keys, uint32_t* bins,
+                              int num_sms, size_t smem_optin, cudaStream_t st) {
   if (a.d == 0 || (a.d % 4) != 0 || !out) return cudaErrorInvalidValue;
   const uint64_t nq = a.queries ? a.nq : a.n;
   if (nq == 0) return cudaSuccess;
   const size_t smem = 32 * static_cast<size_t>(seed_stride4(a.d)) * 16 +
                       2 * kSeedTile * static_cast<size_t>(a.d) * 4;
   if (smem > smem_optin) return cudaErrorInvalidValue;
-  auto kern = k_seed_dists;
+  auto kern = keys ? k_seed_dists<true> : k_seed_dists<false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
@@ -608,7 +633,106 @@ cudaError_t launch_seed_dists(const SearchArgs& a, float* out, int num_sms,
   uint64_t blocks = (nq + kSeedTile - 1) / kSeedTile;
   const uint64_t cap = static_cast<uint64_t>(num_sms) * (per_sm < 1 ? 1 : per_sm);
   if (blocks > cap) blocks = cap;
-  kern<<<static_cast<unsigned>(blocks), 32 * kSeedWarps, smem, st>>>(a, out);
+  kern<<<static_cast<unsigned>(blocks), 32 * kSeedWarps, smem, st>>>(
+      a, out, keys, bins, keys_per_segment(a.seg_count));
+  return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------------
+// Relocation.  A point's lists hold points near it, and points near each other share their nearest
+// seeds.  Working on a copy of the base sorted by (nearest, second nearest seed) puts the rows that
+// neighbouring warps gather next to each other: fewer DRAM rows, fewer address translations, more
+// cache hits.  Nothing in the search or the prunes depends on the numbering (ties go by position);
+// the reverse lists, which keep the first sources by id, are sorted by original id.
+// Whole builds on the caller's rows -> relocated: 1M x 512 cosine (L = 96) 758 -> 491 ms, 300k x 512
+// 199 -> 147, 1M x 200 72.3 -> 69.5, 100k x 200 8.80 -> 8.53, 50k x 200 4.97 -> 4.81, 20k x 200
+// 2.53 -> 2.57, 10k x 512 4.33 -> 4.53: below 32 MB the base stays in L2 and the extra passes cost
+// more than they give.  The copy doubles the base's memory, so it stops at 32 GB (and where the
+// workspace cannot be allocated).
+uint32_t reloc_keys(uint64_t n, uint32_t d, uint32_t seg_count) {
+  constexpr uint64_t kMin = 32ull << 20, kMax = 32ull << 30;  // bytes of the base
+  if (n * d * 4 < kMin || n * d * 4 > kMax || seg_count > 2048) return 0;
+  const uint32_t k = (seg_count ? seg_count : 1u) * keys_per_segment(seg_count);
+  return (k + 1023u) / 1024u * 1024u;
+}
+
+// Counts -> starting places, in place (one block; count a multiple of 1024).
+__global__ void __launch_bounds__(1024) k_reloc_starts(uint32_t* __restrict__ bins,
+                                                       uint32_t count) {
+  __shared__ uint32_t ws[32];
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  uint32_t carry = 0;
+  for (uint32_t b0 = 0; b0 < count; b0 += 1024) {
+    const uint32_t v = bins[b0 + threadIdx.x];
+    uint32_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, x, o);
+      if (lane >= static_cast<uint32_t>(o)) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    const uint32_t w = ws[lane];
+    uint32_t all = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, all, o);
+      if (lane >= static_cast<uint32_t>(o)) all += y;
+    }
+    const uint32_t before = __shfl_sync(kFull, all - w, static_cast<int>(warp));
+    bins[b0 + threadIdx.x] = carry + before + x - v;
+    carry += __shfl_sync(kFull, all, 31);
+    __syncthreads();
+  }
+}
+
+__global__ void k_reloc_place(const uint32_t* __restrict__ keys, uint64_t n,
+                              uint32_t* __restrict__ cursor, uint32_t* __restrict__ order,
+                              uint32_t* __restrict__ place) {
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += stride) {
+    const uint32_t at = atomicAdd(cursor + keys[i], 1u);
+    order[at] = static_cast<uint32_t>(i);
+    place[i] = at;
+  }
+}
+
+// One warp per row: d / 4 + 8 float4 copies, coalesced on both sides.
+__global__ void __launch_bounds__(256) k_reloc_rows(const float4* __restrict__ base, uint64_t n,
+                                                    uint32_t d4, const float4* __restrict__ seeds,
+                                                    const uint32_t* __restrict__ order,
+                                                    float4* __restrict__ out_base,
+                                                    float4* __restrict__ out_seeds) {
+  const uint32_t lane = lane_id();
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * 8;
+  for (uint64_t i = blockIdx.x * 8ull + (threadIdx.x >> 5); i < n; i += nw) {
+    const uint64_t o = order[i];
+#pragma unroll 4
+    for (uint32_t c = lane; c < d4; c += 32) out_base[i * d4 + c] = __ldg(base + o * d4 + c);
+    if (lane < 8) out_seeds[i * 8 + lane] = __ldg(seeds + o * 8 + lane);
+  }
+}
+
+cudaError_t launch_reloc_order(const uint32_t* keys, uint64_t n, uint32_t* bins, uint32_t nkeys,
+                               uint32_t* order, uint32_t* place, int num_sms, cudaStream_t st) {
+  k_reloc_starts<<<1, 1024, 0, st>>>(bins, nkeys);
+  uint64_t blocks = (n + 255) / 256;
+  const uint64_t cap = static_cast<uint64_t>(num_sms) * 8;
+  if (blocks > cap) blocks = cap;
+  k_reloc_place<<<static_cast<unsigned>(blocks), 256, 0, st>>>(keys, n, bins, order, place);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_reloc_rows(const float* base, uint64_t n, uint32_t d, const float* seeds,
+                              const uint32_t* order, float* out_base, float* out_seeds,
+                              int num_sms, cudaStream_t st) {
+  uint64_t blocks = (n + 7) / 8;
+  const uint64_t cap = static_cast<uint64_t>(num_sms) * 8;
+  if (blocks > cap) blocks = cap;
+  k_reloc_rows<<<static_cast<unsigned>(blocks), 256, 0, st>>>(
+      reinterpret_cast<const float4*>(base), n, d / 4, reinterpret_cast<const float4*>(seeds),
+      order, reinterpret_cast<float4*>(out_base), reinterpret_cast<float4*>(out_seeds));
   return cudaGetLastError();
 }
 

@@ -40,7 +40,7 @@ namespace {
 constexpr uint32_t kGtCap = 1024;          // candidates per query
 constexpr uint32_t kGtErrRange = 1u << 4;  // a value beyond the FP16 range
 constexpr uint32_t kGtErrFinal = 1u << 6;  // a query kept more candidates than kGtCap
-constexpr int kFinalWarps = 2;
+constexpr uint32_t kGtShort = 256;         // lists of the final pass's common kernel
 
 __device__ __forceinline__ float key_value(uint64_t key) {  // inverse of desc_key's value part
   const uint32_t o = ~static_cast<uint32_t>(key >> 32);
@@ -51,12 +51,6 @@ __device__ __forceinline__ float key_value(uint64_t key) {  // inverse of desc_k
 // descending value, then ascending id, as an ascending 64-bit key
 __device__ __forceinline__ uint64_t desc_key(float v, uint32_t id) {
   return (static_cast<uint64_t>(~order_key(v)) << 32) | id;
-}
-
-__device__ __forceinline__ uint64_t desc_key64(double v) {  // descending double
-  const uint64_t u = static_cast<uint64_t>(__double_as_longlong(v + 0.0));
-  const uint64_t o = (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-  return ~o;
 }
 
 // FP16 copy of rows x d FP32 values with row stride dp >= d (zeros in the padding), and per row
@@ -132,10 +126,10 @@ __global__ void k_gt_band(const float* __restrict__ qn, const float* __restrict_
 
 // ---------------------------------------------------------------- selection helpers
 
-// Sorts buf[0 .. cnt) (desc value, asc id); returns the k-th largest value (or -inf when
-// cnt < k) and keeps in buf the prefix with value >= that - band; *cnt updated.
+// Sorts buf[0 .. cnt) (desc value, asc id) and keeps the prefix with value >= the k-th largest
+// value - band (all of it when cnt < k); cnt updated.
 template <int E>
-__device__ float compact_sorted(uint64_t* buf, uint32_t& cnt, uint32_t k, float band) {
+__device__ void compact_sorted(uint64_t* buf, uint32_t& cnt, uint32_t k, float band) {
   const uint32_t lane = lane_id();
   uint64_t key[E];
 #pragma unroll
@@ -165,14 +159,18 @@ __device__ float compact_sorted(uint64_t* buf, uint32_t& cnt, uint32_t k, float 
   }
   __syncwarp();
   cnt = keep;
-  return theta;
 }
 
-__device__ float compact_any(uint64_t* buf, uint32_t& cnt, uint32_t k, float band) {
-  if (cnt <= 128) return compact_sorted<4>(buf, cnt, k, band);
-  if (cnt <= 256) return compact_sorted<8>(buf, cnt, k, band);
-  if (cnt <= 512) return compact_sorted<16>(buf, cnt, k, band);
-  return compact_sorted<32>(buf, cnt, k, band);
+template <uint32_t CAP>
+__device__ void compact_any(uint64_t* buf, uint32_t& cnt, uint32_t k, float band) {
+  if (cnt <= 128)
+    compact_sorted<4>(buf, cnt, k, band);
+  else if (CAP <= 256 || cnt <= 256)
+    compact_sorted<8>(buf, cnt, k, band);
+  else if (cnt <= 512)
+    compact_sorted<16>(buf, cnt, k, band);
+  else
+    compact_sorted<32>(buf, cnt, k, band);
 }
 
 // The k-th smallest of key(0 .. cnt-1) (32-bit keys), by a four-pass 8-bit radix select with a
@@ -235,106 +233,236 @@ struct GtArgs {
   const uint64_t* cand;      // rows x kGtCap keys (desc_key), two halves of kGtCap / 2
   const uint32_t* cand_cnt;  // rows x 2
   const float* band;         // rows
+  const float *qn, *qe;      // rows: upper bounds of |q^| and |q - q^|
+  const uint32_t* xmax;      // bits of max |x^| and max |x - x^|
   uint32_t* out;             // rows x k
-  uint32_t* status;
 };
 
-// Exact FP64 scores of the candidates c = buf[0 .. cnt), sorted by (score desc, id asc); the
-// first k ids go to out (tomb past cnt).
-template <int E>
-__device__ void rescore_write(const GtArgs& a, uint64_t row, const uint64_t* buf, uint32_t cnt,
-                              uint32_t* ids_s) {
-  const uint32_t lane = lane_id();
-  const float* q = a.queries + row * a.d;
-  uint64_t key[E];
-  uint32_t id[E];
-#pragma unroll
-  for (int s = 0; s < E; s++) {
-    const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
-    key[s] = ~0ull;
-    id[s] = kTomb;
-    if (i < cnt) {
-      const uint32_t x = static_cast<uint32_t>(buf[i]);
-      const float* xr = a.base + static_cast<uint64_t>(x) * a.d;
-      double acc = 0.0;
-      for (uint32_t j = 0; j < a.d; j++)
-        acc = fma(static_cast<double>(q[j]), static_cast<double>(xr[j]), acc);
-      key[s] = desc_key64(acc);
-      id[s] = x;
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* p) {
+  if constexpr (VEC) return __ldg(reinterpret_cast<const float4*>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
+// FP32 inner products of the query (shared memory) with the rows of ids buf[0 .. cnt) (low words):
+// eight lanes per row, four rows per load, two loads in flight per step.  Lane m of a group sums
+// elements 32 k + 4 m + j in four chains, so a score carries at most d / 32 + 6 roundings.  The
+// keys are replaced by (score descending, id).
+template <bool VEC>
+__device__ __forceinline__ void score_candidates(const float* __restrict__ base, uint32_t d,
+                                                 const float* q_s, uint64_t* buf, uint32_t cnt) {
+  const uint32_t lane = lane_id(), g = lane >> 3, m = lane & 7u;
+  for (uint32_t c0 = 0; c0 < cnt; c0 += 8) {
+    const uint32_t i0 = min(c0 + g, cnt - 1), i1 = min(c0 + 4 + g, cnt - 1);
+    const uint32_t id0 = static_cast<uint32_t>(buf[i0]), id1 = static_cast<uint32_t>(buf[i1]);
+    const float* r0 = base + static_cast<uint64_t>(id0) * d;
+    const float* r1 = base + static_cast<uint64_t>(id1) * d;
+    float p0[4] = {0.f, 0.f, 0.f, 0.f}, p1[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (uint32_t c = 4u * m; c < d; c += 32) {
+      const float4 x = load4<VEC>(r0 + c), y = load4<VEC>(r1 + c);
+      const float4 u = *reinterpret_cast<const float4*>(q_s + c);
+      p0[0] = fmaf(u.x, x.x, p0[0]);
+      p0[1] = fmaf(u.y, x.y, p0[1]);
+      p0[2] = fmaf(u.z, x.z, p0[2]);
+      p0[3] = fmaf(u.w, x.w, p0[3]);
+      p1[0] = fmaf(u.x, y.x, p1[0]);
+      p1[1] = fmaf(u.y, y.y, p1[1]);
+      p1[2] = fmaf(u.z, y.z, p1[2]);
+      p1[3] = fmaf(u.w, y.w, p1[3]);
     }
+    // lanes with m < 4 reduce the first row, the others the second
+    const float s0 = (p0[0] + p0[1]) + (p0[2] + p0[3]), s1 = (p1[0] + p1[1]) + (p1[2] + p1[3]);
+    const bool up = (m & 4u) != 0;
+    float t = (up ? s1 : s0) + __shfl_xor_sync(kFull, up ? s0 : s1, 4);
+    t += __shfl_xor_sync(kFull, t, 2);
+    t += __shfl_xor_sync(kFull, t, 1);
+    __syncwarp();
+    if (m == 0 && c0 + g < cnt) buf[c0 + g] = desc_key(t, id0);
+    if (m == 4 && c0 + 4 + g < cnt) buf[c0 + 4 + g] = desc_key(t, id1);
+    __syncwarp();
   }
-  warp_sort_kv<E>(key, id);
-  // equal FP64 scores (duplicate vectors): ascending id inside each run
+}
+
+template <int E>
+__device__ __forceinline__ void sort_keys(uint64_t* buf, uint32_t cnt) {
+  const uint32_t lane = lane_id();
+  uint64_t key[E];
 #pragma unroll
   for (int s = 0; s < E; s++) {
     const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
-    if (i < cnt) ids_s[i] = id[s];
-  }
-  bool tie = false;
-#pragma unroll
-  for (int s = 0; s < E; s++) {
-    const uint64_t up = __shfl_up_sync(kFull, key[s], 1);
-    const uint64_t wrap = s > 0 ? __shfl_sync(kFull, key[s > 0 ? s - 1 : 0], 31) : ~0ull;
-    const uint64_t prev = lane == 0 ? wrap : up;
-    const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
-    tie |= i > 0 && i < cnt && prev == key[s];
+    key[s] = i < cnt ? buf[i] : ~0ull;
   }
   __syncwarp();
-  if (__any_sync(kFull, tie)) {
-    uint64_t* ks = const_cast<uint64_t*>(buf);  // reuse as keys
+  warp_sort_u64<E>(key);
 #pragma unroll
-    for (int s = 0; s < E; s++) {
-      const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
-      if (i < cnt) ks[i] = key[s];
-    }
-    __syncwarp();
-    if (lane == 0) {  // insertion sort by id inside runs of equal keys
-      for (uint32_t i = 1; i < cnt; i++) {
-        uint32_t j = i;
-        while (j > 0 && ks[j - 1] == ks[j] && ids_s[j - 1] > ids_s[j]) {
-          const uint32_t t = ids_s[j];
-          ids_s[j] = ids_s[j - 1];
-          ids_s[j - 1] = t;
-          j--;
-        }
-      }
-    }
-    __syncwarp();
+  for (int s = 0; s < E; s++) {
+    const uint32_t i = static_cast<uint32_t>(s) * 32u + lane;
+    if (i < cnt) buf[i] = key[s];
   }
-  uint32_t* o = a.out + row * a.k;
-  for (uint32_t i = lane; i < a.k; i += 32) o[i] = i < cnt ? ids_s[i] : kTomb;
   __syncwarp();
 }
 
-// One warp per query: its candidates (those with s^ >= theta - 2 E_q), then the ones with
-// s^ >= t_k - 2 E_q, re-scored in FP64 and sorted.
-__global__ void __launch_bounds__(kFinalWarps * 32) k_gt_final(GtArgs a) {
-  __shared__ uint64_t buf_all[kFinalWarps][kGtCap];
-  __shared__ uint32_t ids_all[kFinalWarps][kGtCap];
-  uint64_t* buf = buf_all[threadIdx.x >> 5];
-  uint32_t* ids_s = ids_all[threadIdx.x >> 5];
-  const uint32_t lane = lane_id();
-  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * kFinalWarps;
-  for (uint64_t row = blockIdx.x * static_cast<uint64_t>(kFinalWarps) + (threadIdx.x >> 5);
-       row < a.rows; row += nw) {
+template <uint32_t CAP>
+__device__ void sort_any(uint64_t* buf, uint32_t cnt) {
+  if (cnt <= 32)
+    sort_keys<1>(buf, cnt);
+  else if (cnt <= 64)
+    sort_keys<2>(buf, cnt);
+  else if (cnt <= 128)
+    sort_keys<4>(buf, cnt);
+  else if (CAP <= 256 || cnt <= 256)
+    sort_keys<8>(buf, cnt);
+  else if (cnt <= 512)
+    sort_keys<16>(buf, cnt);
+  else
+    sort_keys<32>(buf, cnt);
+}
+
+// Warps (queries in flight) per block of the final pass, and its shared memory: per warp the keys,
+// FP64 scores, link bits and the query, then the block's list of runs to settle.
+template <bool LONG>
+struct Final {
+  static constexpr uint32_t kCap = LONG ? kGtCap : kGtShort;
+  static constexpr uint32_t kWarps = LONG ? 4 : 8;
+  static constexpr uint32_t kWarpBytes = kCap * 16 + kCap / 8;
+  static size_t smem(uint32_t d) { return kWarps * (kWarpBytes + 4ull * d + kCap * 2); }
+};
+
+// One warp per query with at most kGtShort candidates (LONG: with more): the candidates, which hold
+// the true top k, in the order of their FP64 inner products.  An FP32 score s is within E32 of the
+// exact product and of its FP64 chain, E32 = (d / 32 + 9) 2^-24 |q| max|x|; candidates sorted by s
+// whose neighbours lie farther than 2 E32 away are thereby in place.  Runs of closer ones that
+// begin before place k are scored by the FP64 chain (ascending element order) and ordered by
+// (score desc, id asc) inside their run.
+// About three candidates of 140 are in such runs.  A warp-wide FP64 instruction occupies the FP64
+// units equally long for three lanes as for 32, so the block's warps pool their runs and one lane
+// takes one candidate.  250k queries of 200 floats, k = 128: 47 ms with an FP64 chain for every
+// candidate, 17 ms with each warp settling its own runs, and 5.4 ms this way (row gathers and the
+// sort).
+template <bool LONG, bool VEC>
+__global__ void __launch_bounds__(Final<LONG>::kWarps * 32) k_gt_final(GtArgs a) {
+  extern __shared__ __align__(16) unsigned char final_smem[];
+  using F = Final<LONG>;
+  constexpr uint32_t CAP = F::kCap;
+  __shared__ uint32_t listed;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  const uint32_t stride = F::kWarpBytes + 4 * a.d;
+  unsigned char* mine = final_smem + warp * stride;
+  uint64_t* buf = reinterpret_cast<uint64_t*>(mine);
+  double* exact = reinterpret_cast<double*>(mine + CAP * 8);
+  uint32_t* links = reinterpret_cast<uint32_t*>(mine + CAP * 16);
+  float* q_s = reinterpret_cast<float*>(mine + F::kWarpBytes);
+  uint16_t* list = reinterpret_cast<uint16_t*>(final_smem + F::kWarps * stride);  // warp, place
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * F::kWarps;
+  const float xm = __fadd_ru(__uint_as_float(a.xmax[0]), __uint_as_float(a.xmax[1]));
+  const float coef = static_cast<float>(a.d / 32u + 10u) * 5.9604645e-08f;  // one spare rounding
+  if (threadIdx.x == 0) listed = 0;
+  for (uint64_t row0 = blockIdx.x * static_cast<uint64_t>(F::kWarps); row0 < a.rows; row0 += nw) {
+    const uint64_t row = row0 + warp;
     // the row's list is two halves of kGtCap / 2, one per half of the columns
-    const uint32_t c0 = min(a.cand_cnt[2 * row], kGtCap / 2);
-    const uint32_t c1 = min(a.cand_cnt[2 * row + 1], kGtCap / 2);
-    const uint64_t* src = a.cand + row * kGtCap;
-    for (uint32_t i = lane; i < c0; i += 32) buf[i] = src[i];
-    for (uint32_t i = lane; i < c1; i += 32) buf[c0 + i] = src[kGtCap / 2 + i];
+    uint32_t c0 = 0, c1 = 0;
+    if (row < a.rows) {
+      c0 = min(a.cand_cnt[2 * row], kGtCap / 2);
+      c1 = min(a.cand_cnt[2 * row + 1], kGtCap / 2);
+    }
     uint32_t cnt = c0 + c1;
+    const bool active = row < a.rows && (cnt > kGtShort) == LONG;
+    if (!__syncthreads_or(active)) continue;
+    auto linked = [&](uint32_t i) { return (links[i / 32] >> (i & 31u)) & 1u; };
+    auto in_run = [&](uint32_t i) { return linked(i) || (i > 0 && linked(i - 1)); };
+    auto run_start = [&](uint32_t i) {
+      while (i > 0 && linked(i - 1)) i--;
+      return i;
+    };
+    bool any = false;
+    if (active) {
+      const uint64_t* src = a.cand + row * kGtCap;
+      const float* q = a.queries + row * a.d;
+      for (uint32_t i = lane; i < c0; i += 32) buf[i] = src[i];
+      for (uint32_t i = lane; i < c1; i += 32) buf[c0 + i] = src[kGtCap / 2 + i];
+      for (uint32_t i = lane; i < a.d; i += 32) q_s[i] = q[i];
+      __syncwarp();
+      if (cnt > 2 * a.k) compact_any<CAP>(buf, cnt, a.k, a.band[row]);  // those >= t_k - band
+      if (cnt) score_candidates<VEC>(a.base, a.d, q_s, buf, cnt);
+      sort_any<CAP>(buf, cnt);
+      const float gap = __fmul_ru(__fmul_ru(2.0f * coef, xm), __fadd_ru(a.qn[row], a.qe[row])) +
+                        1e-37f;
+      for (uint32_t i0 = 0; i0 < cnt; i0 += 32) {  // bit i: candidates i and i + 1 are too close
+        const uint32_t i = i0 + lane;
+        const bool l = i + 1 < cnt && !(key_value(buf[i]) - key_value(buf[i + 1]) > gap);
+        const unsigned w = __ballot_sync(kFull, l);
+        if (lane == 0) links[i0 / 32] = w;
+        any |= w != 0;
+      }
+      __syncwarp();
+      if (any)
+        for (uint32_t i = lane; i < cnt; i += 32)
+          if (in_run(i) && run_start(i) < a.k)
+            list[atomicAdd(&listed, 1u)] = static_cast<uint16_t>(warp * CAP + i);
+    }
+    __syncthreads();
+    const uint32_t total = listed;
+    for (uint32_t t = threadIdx.x; t < total; t += blockDim.x) {
+      const uint32_t w = list[t] / CAP, i = list[t] % CAP;
+      unsigned char* its = final_smem + w * stride;
+      const uint32_t id = static_cast<uint32_t>(reinterpret_cast<const uint64_t*>(its)[i]);
+      const float* xr = a.base + static_cast<uint64_t>(id) * a.d;
+      const float* qr = reinterpret_cast<const float*>(its + F::kWarpBytes);
+      double acc = 0.0;
+#pragma unroll 2
+      for (uint32_t j = 0; j < a.d; j += 4) {
+        const float4 x = load4<VEC>(xr + j);
+        const float4 u = *reinterpret_cast<const float4*>(qr + j);
+        acc = fma(static_cast<double>(u.x), static_cast<double>(x.x), acc);
+        acc = fma(static_cast<double>(u.y), static_cast<double>(x.y), acc);
+        acc = fma(static_cast<double>(u.z), static_cast<double>(x.z), acc);
+        acc = fma(static_cast<double>(u.w), static_cast<double>(x.w), acc);
+      }
+      reinterpret_cast<double*>(its + CAP * 8)[i] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) listed = 0;  // the next use follows the loop's first barrier
+    if (!active) continue;
+    uint32_t* o = a.out + row * a.k;
+    for (uint32_t i = lane; i < cnt; i += 32) {
+      const uint32_t id = static_cast<uint32_t>(buf[i]);
+      uint32_t pos = i;
+      if (any && in_run(i)) {
+        pos = run_start(i);
+        if (pos < a.k) {
+          const double mv = exact[i];
+          for (uint32_t j = pos;; j++) {
+            const double v = exact[j];
+            if (v > mv || (v == mv && static_cast<uint32_t>(buf[j]) < id)) pos++;
+            if (!linked(j)) break;
+          }
+        }
+      }
+      if (pos < a.k) o[pos] = id;
+    }
+    for (uint32_t i = cnt + lane; i < a.k; i += 32) o[i] = kTomb;
     __syncwarp();
-    compact_any(buf, cnt, a.k, a.band[row]);  // candidates >= t_k - band, sorted
-    if (cnt <= 128)
-      rescore_write<4>(a, row, buf, cnt, ids_s);
-    else if (cnt <= 256)
-      rescore_write<8>(a, row, buf, cnt, ids_s);
-    else if (cnt <= 512)
-      rescore_write<16>(a, row, buf, cnt, ids_s);
-    else
-      rescore_write<32>(a, row, buf, cnt, ids_s);
   }
+}
+
+template <bool LONG>
+cudaError_t launch_final(const GtArgs& f, int num_sms, cudaStream_t st) {
+  using F = Final<LONG>;
+  const bool vec = (reinterpret_cast<uintptr_t>(f.base) & 15u) == 0;
+  auto kern = vec ? k_gt_final<LONG, true> : k_gt_final<LONG, false>;
+  const size_t smem = F::smem(f.d);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, F::kWarps * 32, smem);
+  if (e != cudaSuccess) return e;
+  uint64_t blocks = (f.rows + F::kWarps - 1) / F::kWarps;
+  const uint64_t cap = static_cast<uint64_t>(num_sms) * (per_sm < 1 ? 1 : per_sm);
+  if (blocks > cap) blocks = cap;
+  kern<<<static_cast<unsigned>(blocks), F::kWarps * 32, smem, st>>>(f);
+  return cudaGetLastError();
 }
 
 // One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima
@@ -889,10 +1017,14 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
     f.cand = cand;
     f.cand_cnt = cand_cnt;
     f.band = band;
+    f.qn = qn + q0;
+    f.qe = qe + q0;
+    f.xmax = xmax;
     f.out = out + q0 * k;
-    f.status = status;
-    k_gt_final<<<blocks_for(rows, kFinalWarps, num_sms, 16), kFinalWarps * 32, 0, st>>>(f);
-    if ((e = cudaGetLastError()) != cudaSuccess) return -static_cast<int>(e);
+    // most lists are short; the long ones take a kernel with room for them
+    if ((e = launch_final<false>(f, num_sms, st)) != cudaSuccess) return -static_cast<int>(e);
+    if ((e = launch_final<true>(f, num_sms, st)) != cudaSuccess)
+      return -static_cast<int>(e);
     if (diag && q0 == 0) {  // the first query's margin and the base's largest norms
       if ((e = cudaMemcpyAsync(diag, band, 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
         return -static_cast<int>(e);

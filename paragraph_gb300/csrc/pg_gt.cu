@@ -173,58 +173,6 @@ __device__ void compact_any(uint64_t* buf, uint32_t& cnt, uint32_t k, float band
     compact_sorted<32>(buf, cnt, k, band);
 }
 
-// The k-th smallest of key(0 .. cnt-1) (32-bit keys), by a four-pass 8-bit radix select with a
-// 256-bin histogram in shared memory.  Requires cnt >= k.  One warp.
-template <class Key>
-__device__ uint32_t radix_kth(Key key, uint32_t cnt, uint32_t k, uint32_t* hist) {
-  const uint32_t lane = lane_id();
-  uint32_t prefix = 0, mask = 0, rem = k;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (uint32_t b = lane; b < 256; b += 32) hist[b] = 0;
-    __syncwarp();
-    for (uint32_t i = lane; i < cnt; i += 32) {
-      const uint32_t vk = key(i);
-      if ((vk & mask) == prefix) atomicAdd(hist + ((vk >> shift) & 255u), 1u);
-    }
-    __syncwarp();
-    uint32_t local[8], sum = 0;
-#pragma unroll
-    for (int t = 0; t < 8; t++) {
-      local[t] = hist[lane * 8 + t];
-      sum += local[t];
-    }
-    uint32_t incl = sum;  // inclusive scan of the lanes' sums
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(kFull, incl, o);
-      if (lane >= static_cast<uint32_t>(o)) incl += y;
-    }
-    const uint32_t excl = incl - sum;
-    const unsigned owner = __ballot_sync(kFull, excl < rem && rem <= incl);
-    const uint32_t src = static_cast<uint32_t>(__ffs(static_cast<int>(owner)) - 1);
-    uint32_t bin = 0, before = 0;
-    if (lane == src) {
-      uint32_t c = excl;
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        if (c + local[t] >= rem) {
-          bin = lane * 8 + t;
-          before = c;
-          break;
-        }
-        c += local[t];
-      }
-    }
-    bin = __shfl_sync(kFull, bin, src);
-    before = __shfl_sync(kFull, before, src);
-    prefix |= bin << shift;
-    mask |= 255u << shift;
-    rem -= before;
-    __syncwarp();
-  }
-  return prefix;
-}
-
 struct GtArgs {
   const float* base;     // n x d (FP32)
   const float* queries;  // rows x d (FP32, this chunk)
@@ -465,25 +413,140 @@ cudaError_t launch_final(const GtArgs& f, int num_sms, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima
-// (-inf when there are fewer than k groups: every base row is then a candidate).
+// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima (-inf when
+// there are fewer than k groups: every base row is then a candidate).
+// A histogram of kThetaBins equal steps between the row's smallest and largest maximum finds the
+// step that holds the k-th largest; its few maxima are then gathered and ranked.  A step with more
+// than kThetaBins of them (an outlier far above the rest) is divided again.  The maxima spread over
+// the steps, so the shared-memory counters see few collisions and three passes over the row mostly
+// do: 3.4 -> 1.6 ms for 250k rows of 4700 maxima against a radix select, whose first of four
+// histograms collides on the sign and exponent.
+constexpr uint32_t kThetaBins = 512;
+template <bool PAIRS>  // an even number of groups: rows start on 8 bytes
 __global__ void __launch_bounds__(256) k_gt_theta(const float* __restrict__ maxima,
                                                   uint32_t rows, uint32_t groups, uint32_t k,
                                                   const float* __restrict__ band,
                                                   float* __restrict__ lo) {
-  __shared__ uint32_t hist_all[8][256];
+  __shared__ uint32_t hist_all[8][kThetaBins];
+  __shared__ uint32_t fill_all[8];
   uint32_t* hist = hist_all[threadIdx.x >> 5];
+  uint32_t* fill = fill_all + (threadIdx.x >> 5);
+  const uint32_t lane = lane_id();
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * 8;
   for (uint64_t row = blockIdx.x * 8ull + (threadIdx.x >> 5); row < rows; row += nw) {
-    if (groups < k) {
-      if (lane_id() == 0) lo[row] = -INFINITY;
+    const float* m = maxima + row * groups;
+    auto each = [&](auto&& use) {  // every maximum once, eight loads in flight per lane
+      if constexpr (PAIRS) {
+        const float2* m2 = reinterpret_cast<const float2*>(m);
+#pragma unroll 8
+        for (uint32_t i = lane; i < groups / 2; i += 32) {
+          const float2 v = m2[i];
+          use(v.x);
+          use(v.y);
+        }
+      } else {
+#pragma unroll 8
+        for (uint32_t i = lane; i < groups; i += 32) use(m[i]);
+      }
+    };
+    // the finite maxima's range and number (a group past the base's end is -inf)
+    float mn = INFINITY, mx = -INFINITY;
+    uint32_t have = 0;
+    each([&](float v) {
+      if (v > -INFINITY) {
+        mn = fminf(mn, v);
+        mx = fmaxf(mx, v);
+        have++;
+      }
+    });
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+    }
+    have = __reduce_add_sync(kFull, have);
+    if (have < k) {
+      if (lane == 0) lo[row] = -INFINITY;
       continue;
     }
-    const float* m = maxima + row * groups;
-    const uint32_t kv =
-        radix_kth([m](uint32_t i) { return ~order_key(m[i]); }, groups, k, hist);
-    const float theta = key_value(static_cast<uint64_t>(kv) << 32);
-    if (lane_id() == 0) lo[row] = theta - band[row];
+    uint32_t need = k;  // theta's rank among the maxima in [mn, mx]
+    for (;;) {
+      const float scale = static_cast<float>(kThetaBins - 1) / (mx - mn);
+      // equal, or not divisible (a value out of range, which raised its error): all count
+      if (!(mx > mn) || !(scale > 0.0f && scale < INFINITY)) break;
+      const float low = mn, high = mx;
+      auto bin = [&](float v) {  // non-decreasing in v
+        return min(static_cast<uint32_t>((v - low) * scale), kThetaBins - 1);
+      };
+      for (uint32_t b = lane; b < kThetaBins; b += 32) hist[b] = 0;
+      __syncwarp();
+      each([&](float v) {
+        if (v >= low && v <= high) atomicAdd(hist + bin(v), 1u);
+      });
+      __syncwarp();
+      // lane l sums bins from the top: kThetaBins - 1 - 16 l downwards
+      constexpr uint32_t kPer = kThetaBins / 32;
+      uint32_t sum = 0;
+      for (uint32_t t = 0; t < kPer; t++) sum += hist[kThetaBins - 1 - (lane * kPer + t)];
+      uint32_t incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= static_cast<uint32_t>(o)) incl += y;
+      }
+      const uint32_t excl = incl - sum;
+      const unsigned owner = __ballot_sync(kFull, excl < need && need <= incl);
+      const int src = __ffs(static_cast<int>(owner)) - 1;
+      uint32_t at = 0, above = 0, held = 0;
+      if (static_cast<int>(lane) == src) {
+        above = excl;
+        for (uint32_t t = 0; t < kPer; t++) {
+          at = kThetaBins - 1 - (lane * kPer + t);
+          held = hist[at];
+          if (above + held >= need) break;
+          above += held;
+        }
+      }
+      at = __shfl_sync(kFull, at, src);
+      above = __shfl_sync(kFull, above, src);
+      held = __shfl_sync(kFull, held, src);
+      need -= above;
+      __syncwarp();
+      if (held <= kThetaBins) {  // its values in the counters' place; the need-th largest of them
+        float* vals = reinterpret_cast<float*>(hist);
+        if (lane == 0) *fill = 0;
+        __syncwarp();
+        each([&](float v) {
+          if (v >= low && v <= high && bin(v) == at) vals[atomicAdd(fill, 1u)] = v;
+        });
+        __syncwarp();
+        mn = INFINITY;
+        for (uint32_t i = lane; i < held; i += 32) {
+          const float v = vals[i];
+          uint32_t gt = 0, eq = 0;
+          for (uint32_t j = 0; j < held; j++) {
+            gt += vals[j] > v ? 1u : 0u;
+            eq += vals[j] == v ? 1u : 0u;
+          }
+          if (gt < need && need <= gt + eq) mn = v;
+        }
+        for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+        __syncwarp();
+        break;
+      }
+      mn = INFINITY;
+      mx = -INFINITY;
+      each([&](float v) {
+        if (v >= low && v <= high && bin(v) == at) {
+          mn = fminf(mn, v);
+          mx = fmaxf(mx, v);
+        }
+      });
+      for (int o = 16; o > 0; o >>= 1) {
+        mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+        mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+      }
+    }
+    if (lane == 0) lo[row] = mn - band[row];
   }
 }
 
@@ -1004,8 +1067,8 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
     a.status = status;
     if ((e = tc::launch<tc::kMax>(ta, tb, a, num_sms, st)) != cudaSuccess)
       return -static_cast<int>(e);
-    k_gt_theta<<<blocks_for(rows, 8, num_sms, 8), 256, 0, st>>>(maxima, rows, plan.groups, k,
-                                                                band, lo);
+    auto theta = plan.groups % 2 ? k_gt_theta<false> : k_gt_theta<true>;
+    theta<<<blocks_for(rows, 8, num_sms, 8), 256, 0, st>>>(maxima, rows, plan.groups, k, band, lo);
     if ((e = tc::launch<tc::kFilter>(ta, tb, a, num_sms, st)) != cudaSuccess)
       return -static_cast<int>(e);
     GtArgs f{};

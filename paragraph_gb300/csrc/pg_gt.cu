@@ -54,7 +54,9 @@ __device__ __forceinline__ uint64_t desc_key(float v, uint32_t id) {
 }
 
 // FP16 copy of rows x d FP32 values with row stride dp >= d (zeros in the padding), and per row
-// upper bounds of |x^| and |x - x^| (FP64 sums rounded up).
+// upper bounds of |x^| and |x - x^|: FP32 sums of squares with every operation rounded up (the
+// difference x - x^ is exact).  FP64 sums took 2.1 ms for 550k rows of 200 floats, the FP64 units
+// being the limit.
 __global__ void k_half_rows(const float* __restrict__ x, uint64_t rows, uint32_t d, uint32_t dp,
                             __half* __restrict__ h, float* __restrict__ nrm,
                             float* __restrict__ enrm, uint32_t* __restrict__ status) {
@@ -62,7 +64,7 @@ __global__ void k_half_rows(const float* __restrict__ x, uint64_t rows, uint32_t
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
   for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
        r < rows; r += nw) {
-    double a = 0.0, e = 0.0;
+    float a = 0.0f, e = 0.0f;
     bool big = false;
     for (uint32_t i = lane; i < dp; i += 32) {
       if (i >= d) {
@@ -73,19 +75,19 @@ __global__ void k_half_rows(const float* __restrict__ x, uint64_t rows, uint32_t
       big |= !(fabsf(v) <= 65000.0f);  // beyond FP16 range (or NaN)
       const __half hv = __float2half_rn(v);
       h[r * dp + i] = hv;
-      const double fv = static_cast<double>(__half2float(hv));
-      a = fma(fv, fv, a);
-      const double ev = static_cast<double>(v) - fv;
-      e = fma(ev, ev, e);
+      const float fv = __half2float(hv);
+      a = __fmaf_ru(fv, fv, a);
+      const float ev = v - fv;
+      e = __fmaf_ru(ev, ev, e);
     }
     for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(kFull, a, o);
-      e += __shfl_xor_sync(kFull, e, o);
+      a = __fadd_ru(a, __shfl_xor_sync(kFull, a, o));
+      e = __fadd_ru(e, __shfl_xor_sync(kFull, e, o));
     }
     if (__any_sync(kFull, big) && lane == 0) raise_error(status, kGtErrRange);
     if (lane == 0) {
-      nrm[r] = __double2float_ru(sqrt(a) * (1.0 + 1e-12));
-      enrm[r] = __double2float_ru(sqrt(e) * (1.0 + 1e-12));
+      nrm[r] = __fsqrt_ru(a);
+      enrm[r] = __fsqrt_ru(e);
     }
   }
 }

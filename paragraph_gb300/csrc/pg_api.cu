@@ -637,7 +637,7 @@ int ensure_ws2(pg_handle h, size_t bytes) {
 }
 
 struct SupLayout {
-  size_t claim, plist, pcnt, indeg, offs, tiles, cursor, edges, rev, rnum, total;
+  size_t claim, plist, pcnt, indeg, offs, tiles, cursor, edges, rev, rnum, queue, total;
 };
 
 SupLayout sup_layout(uint64_t n, uint64_t q, uint32_t m_nn) {
@@ -659,6 +659,7 @@ SupLayout sup_layout(uint64_t n, uint64_t q, uint32_t m_nn) {
   l.edges = take(q * m_nn * 4);
   l.rev = take(n * maxdeg * 4);
   l.rnum = take(n * 4);
+  l.queue = take(pg::roar_queue_bytes(std::max(n, q)));
   l.total = o;
   return l;
 }
@@ -704,6 +705,7 @@ int enqueue_match_sup(pg_handle h, const float* base, uint64_t n, uint32_t d, co
   a.rnum = rnum;
   a.out = out;
   a.cnt = cnt;
+  a.queue = reinterpret_cast<uint32_t*>(w + lay.queue);
   a.status = h->d_status;
   PG_CUDA(pg::launch_sup_claim(gt, q, gt_k, topn, n, claim, h->num_sms, s));
   PG_CUDA(cudaMemsetAsync(a.indeg, 0, n * 4, s));
@@ -724,11 +726,13 @@ int finish(pg_handle h) {
   return status_to_error(*h->h_status);
 }
 
+// The queue takes the start of the workspace: callers have ensured roar_queue_bytes(n) of it.
 pg::FusionArgs fusion_args(pg_handle h, const float* base, uint64_t n, uint32_t d) {
   pg::FusionArgs a{};
   a.base = base;
   a.n = n;
   a.d = d;
+  a.queue = reinterpret_cast<uint32_t*>(h->ws);
   a.status = h->d_status;
   return a;
 }
@@ -1402,6 +1406,8 @@ int pg_fusion_nn(pg_handle h, const float* d_base, uint64_t n, uint32_t d, uint3
   if (!aligned16(d_base)) return fail(PG_EINVAL, "base must be 16-byte aligned");
   std::lock_guard<std::mutex> lk(h->mu);
   PG_CUDA(cudaSetDevice(h->device));
+  int rc = ensure_ws(h, pg::roar_queue_bytes(n));
+  if (rc) return rc;
   PG_CUDA(cudaMemsetAsync(h->d_status, 0, 4, h->stream));
   pg::FusionArgs a = fusion_args(h, d_base, n, d);
   a.sup = d_sup;
@@ -1432,6 +1438,8 @@ int pg_fusion_final(pg_handle h, const float* d_base, uint64_t n, uint32_t d,
   if (!aligned16(d_base)) return fail(PG_EINVAL, "base must be 16-byte aligned");
   std::lock_guard<std::mutex> lk(h->mu);
   PG_CUDA(cudaSetDevice(h->device));
+  int rc = ensure_ws(h, pg::roar_queue_bytes(n));
+  if (rc) return rc;
   PG_CUDA(cudaMemsetAsync(h->d_status, 0, 4, h->stream));
   pg::FusionArgs a = fusion_args(h, d_base, n, d);
   a.bip = d_bip_ids;
@@ -1506,6 +1514,8 @@ int build_index_locked(pg_handle h, const pg_params* p, const float* d_base, uin
     if (rc) return rc;
   }
   PG_CUDA(cudaEventRecord(h->ev[11], s));
+  rc = ensure_ws(h, pg::roar_queue_bytes(n));  // the build's workspace is larger: no allocation
+  if (rc) return rc;
   pg::FusionArgs a = fusion_args(h, d_base, n, d);
   a.sup = sup;
   a.sup_cnt = supc;

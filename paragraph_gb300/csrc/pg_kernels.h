@@ -103,6 +103,7 @@ struct SupArgs {  // one MatchSup round
   const uint32_t* rnum;   // n
   uint32_t* out;          // n x m_nn
   uint32_t* cnt;          // n
+  uint32_t* queue;        // roar_queue_bytes(max(n, q)): work for the one-block-per-node kernels
   uint32_t* status;
 };
 
@@ -127,9 +128,11 @@ struct FusionArgs {
   uint32_t* out;   // n x out_stride
   uint32_t* cnt;   // n
   uint32_t out_stride;
+  uint32_t* queue;  // roar_queue_bytes(n): work for the one-block-per-node kernels
   uint32_t* status;
 };
 
+inline size_t roar_queue_bytes(uint64_t nodes) { return (nodes + 2) * 4; }
 bool roar_supported(uint32_t d, uint32_t m);
 uint32_t roar_capacity();
 cudaError_t launch_sup_claim(const uint32_t* gt, uint64_t q, uint32_t gt_k, uint32_t topn,

@@ -70,7 +70,8 @@ size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 struct Layout {
   size_t winner, pruned, pruned_num, indeg, offs, tile_sums, cursor, edges, rev, rev_num, sres,
-      proj, graph, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place, total;
+      proj, graph, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place,
+      pruned_dist, rev_dist, queue, total;
 };
 
 Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_t L,
@@ -89,9 +90,12 @@ Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_
   l.offs = take((n + 1) * 4);
   l.tile_sums = take(((n + pg::kScanTileElems - 1) / pg::kScanTileElems + 1) * 4);
   l.cursor = take(n * 4);
-  l.edges = take(n * pmax * 4);
+  l.edges = take(n * pmax * 8);
   l.rev = take(n * rmax * 4);
   l.rev_num = take(n * 4);
+  l.pruned_dist = take(n * pmax * 4);
+  l.rev_dist = take(n * rmax * 4);
+  l.queue = take((n + 2) * 4);
   l.sres = take(n * L * 4);
   l.proj = take(n * proj_deg * 4);
   l.graph = take(n * degree * 4);
@@ -325,6 +329,9 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   uint32_t* edges = reinterpret_cast<uint32_t*>(w + lay.edges);
   uint32_t* rev = reinterpret_cast<uint32_t*>(w + lay.rev);
   uint32_t* rnum = reinterpret_cast<uint32_t*>(w + lay.rev_num);
+  float* pdist = reinterpret_cast<float*>(w + lay.pruned_dist);
+  float* rdist = reinterpret_cast<float*>(w + lay.rev_dist);
+  uint32_t* queue = reinterpret_cast<uint32_t*>(w + lay.queue);
   uint32_t* sres = reinterpret_cast<uint32_t*>(w + lay.sres);
   uint32_t* proj = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rproj)
                    : proj_out ? proj_out : reinterpret_cast<uint32_t*>(w + lay.proj);
@@ -407,6 +414,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     pa.strict = 0;
     pa.pruned = pruned;
     pa.pruned_num = pnum;
+    pa.pruned_dist = pdist;
     pa.indeg = indeg;
     pa.sorted = nullptr;
     pa.evals = cnt + C_PROJ_PRUNE;
@@ -417,8 +425,9 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     pa.place = place;
     PG_CUDA(pg::launch_prune_reverse(pa, true, sms, s));
     PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->proj_pruned, n, indeg, offs, tsum, cursor, edges,
-                                   sms, s, 0, order));
-    PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->proj_reverse, rev, rnum, sms, s, place));
+                                   sms, s, 0, order, pdist));
+    PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->proj_reverse, rev, rnum, sms, s, place,
+                                     rdist));
     // K3 phase-1 merge -> projection graph
     pg::MergeArgs ma{};
     ma.base = rows;
@@ -430,6 +439,9 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     ma.reverse = rev;
     ma.reverse_num = rnum;
     ma.r = p->proj_reverse;
+    ma.pruned_dist = pdist;
+    ma.reverse_dist = rdist;
+    ma.queue = queue;
     ma.degree = p->proj_degree;
     ma.strict = 0;
     ma.out = proj;
@@ -481,6 +493,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       pr.strict = 1;
       pr.pruned = pruned;
       pr.pruned_num = pnum;
+      pr.pruned_dist = pdist;
       pr.indeg = indeg;
       pr.sorted = nullptr;
       pr.evals = cnt + C_PRUNE + r;
@@ -496,8 +509,9 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       } else
         PG_CUDA(pg::launch_prune_reverse(pr, false, sms, s));
       PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->degree, n, indeg, offs, tsum, cursor, edges,
-                                     sms, s, 0, order));
-      PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->link_reverse, rev, rnum, sms, s, place));
+                                     sms, s, 0, order, pdist));
+      PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->link_reverse, rev, rnum, sms, s, place,
+                                       rdist));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[3 + 3 * r], s));
       pg::MergeArgs mr{};
       mr.base = rows;
@@ -509,6 +523,11 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       mr.reverse = rev;
       mr.reverse_num = rnum;
       mr.r = p->link_reverse;
+      mr.pruned_dist = pdist;
+      mr.reverse_dist = rdist;
+      mr.own_strict = 1;
+      mr.norms = screened ? norms : nullptr;
+      mr.queue = queue;
       mr.degree = p->degree;
       mr.strict = 1;
       mr.out = link;
@@ -1089,8 +1108,11 @@ int pg_merge_prune(pg_handle h, const float* d_base, uint64_t n, uint32_t d,
   std::lock_guard<std::mutex> lk(h->mu);
   PG_CUDA(cudaSetDevice(h->device));
   cudaStream_t s = h->stream;
+  const int rc = ensure_ws(h, (n + 2) * 4);
+  if (rc) return rc;
   PG_CUDA(cudaMemsetAsync(h->d_counters, 0, 8, s));
   pg::MergeArgs a{};
+  a.queue = reinterpret_cast<uint32_t*>(h->ws);
   a.base = d_base;
   a.n = n;
   a.d = d;

@@ -30,7 +30,7 @@ __device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
 }
 
 // Rows of at least this many floats (1 KB) are read with 256-bit loads by the exact chains of the
-// plain prune and the merges when 32-byte aligned (their launchers pick the WIDE kernels): such
+// prunes and the merges when 32-byte aligned (their launchers pick the WIDE kernels): such
 // rows mostly come from DRAM, where half the load requests pay (measured at 1M x 512: merges
 // 251 -> 190 ms per build); the shorter rows of the L2-resident 1M x 200 workload were measured
 // faster with the float4 kernels.
@@ -211,8 +211,8 @@ __device__ __forceinline__ void warp_sort_u64(uint64_t (&key)[E]) {
 }
 
 // Merge stages only (the input is bitonic): sorts ascending in log2(32E) steps.
-template <int E>
-__device__ __forceinline__ void warp_bitonic_merge_u32(uint32_t (&key)[E]) {
+template <int E, class Key>
+__device__ __forceinline__ void warp_bitonic_merge(Key (&key)[E]) {
   const uint32_t lane = threadIdx.x & 31u;
   constexpr uint32_t n = 32u * E;
 #pragma unroll
@@ -223,17 +223,17 @@ __device__ __forceinline__ void warp_bitonic_merge_u32(uint32_t (&key)[E]) {
       for (int s = 0; s < E; s++) {
         const int s2 = s ^ static_cast<int>(js);
         if (s2 > s) {
-          const uint32_t a = key[s], b = key[s2];
-          key[s] = min(a, b);
-          key[s2] = max(a, b);
+          const Key a = key[s], b = key[s2];
+          key[s] = a < b ? a : b;
+          key[s2] = a < b ? b : a;
         }
       }
     } else {
       const bool lower = (lane & j) == 0;
 #pragma unroll
       for (int s = 0; s < E; s++) {
-        const uint32_t o = __shfl_xor_sync(kFull, key[s], j);
-        key[s] = lower ? min(key[s], o) : max(key[s], o);
+        const Key o = __shfl_xor_sync(kFull, key[s], j);
+        key[s] = lower == (o < key[s]) ? o : key[s];
       }
     }
   }

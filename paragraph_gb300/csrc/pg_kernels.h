@@ -18,6 +18,7 @@ struct PruneArgs {
   int strict;
   uint32_t* pruned;        // n x p
   uint32_t* pruned_num;    // n
+  float* pruned_dist;      // optional n x p: the kept entries' distances (NaN: not a chain's)
   uint32_t* indeg;         // n, incremented per kept edge (reverse in-degree)
   uint32_t* sorted;        // optional n x c: candidate rows after the sort
   unsigned long long* evals;
@@ -49,6 +50,14 @@ struct MergeArgs {
   const uint32_t* reverse;
   const uint32_t* reverse_num;
   uint32_t r;
+  // builds: the lists' distances (both or neither), NaN where none is known
+  const float* pruned_dist;
+  const float* reverse_dist;
+  int own_strict;  // the pruned lists are a strict prune's, with these distances
+  // screened builds: launch_screen_norms' bounds; the tests are decided from FP32 inner products in
+  // another order, the exact chain inside their error bound
+  const float2* norms;
+  uint32_t* queue;  // n + 2 words: nodes with long lists
   uint32_t degree;
   int strict;
   uint32_t* out;  // n x degree
@@ -197,12 +206,15 @@ cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_nu
                                uint64_t n, const uint32_t* indeg, uint32_t* offs,
                                uint32_t* tile_sums, uint32_t* cursor, uint32_t* edges,
                                int num_sms, cudaStream_t st, uint64_t rows = 0,
-                               const uint32_t* order = nullptr);
+                               const uint32_t* order = nullptr,
+                               const float* pruned_dist = nullptr);
+// With pruned_dist / rev_dist every edge carries its distance (edges: 8 bytes each).
 // With order / place (relocated builds) the edges hold original ids, which decide which sources a
 // list keeps and their sequence, and the lists hold places.
 cudaError_t launch_reverse_lists(const uint32_t* offs, const uint32_t* edges, uint64_t n,
                                  uint32_t r, uint32_t* rev, uint32_t* rev_num, int num_sms,
-                                 cudaStream_t st, const uint32_t* place = nullptr);
+                                 cudaStream_t st, const uint32_t* place = nullptr,
+                                 float* rev_dist = nullptr);
 cudaError_t launch_merge_prune(const MergeArgs& a, int num_sms, cudaStream_t st);
 // bytes (a multiple of 16, both pointers 16-byte aligned) from src to dst by a kernel: used with
 // pinned host memory mapped into the device address space (cudaHostGetDevicePointer).

@@ -428,6 +428,8 @@ __global__ void __launch_bounds__(kTile, S == 2 ? 4 : 3) k_prune_tc(const PruneA
       }
       if (my_kept != kNone) {
         a.pruned[b * a.p + my_kept] = x;
+        if (a.pruned_dist)  // a NaN when the list held no chain's distance (the node itself)
+          a.pruned_dist[b * a.p + my_kept] = valid ? dist : __uint_as_float(0x7FFFFFFFu);
         atomicAdd(a.indeg + x, 1u);
       }
     }

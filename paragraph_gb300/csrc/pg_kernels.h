@@ -86,8 +86,8 @@ struct SearchArgs {
   const float* queries;
   uint64_t nq;
   uint32_t out_width;  // ids written per query: L for link rounds, top-k for a query search
-  // launch shape (results do not depend on it): candidate rows scored per pass (8 or 16, Km = 32
-  // kernel) and a cap on resident search warps per SM; 0 = defaults
+  // launch shape (results do not depend on it): candidate rows scored per pass (16: the kernels for
+  // few queries, Km = 32) and a cap on resident search warps per SM; 0 = defaults
   uint32_t rows;
   uint32_t max_blocks_per_sm;
   // optional (n or nq) x 32: each query's distances to its 32 seeds from launch_seed_dists (the

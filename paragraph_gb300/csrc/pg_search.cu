@@ -69,11 +69,11 @@ __device__ __forceinline__ void hash_clear(uint32_t* t, uint32_t slots) {
 //     earlier scheme) is issued lane by lane and held 6-16 KB of shared memory per warp;
 //   * 32-bit keys, one pass over the entering candidates only, and the same ranks for the output
 //     instead of two 64-element sorting networks per query;
-//   * registers held to 80-88 (21-24 warps per SM).  For rows over 256 floats the query stays in
-//     shared memory and four K steps are in flight.
-// Both rounds at 1M x 200, Km = 32: 25.5 + 22.5 -> 18.2 + 15.1 ms; 300k x 512, Km = 64:
-// 38 + 59.4 -> 23.3 + 58.5 ms (DRAM-bound); 400k x 512, Km = 32: 6.6 + 10.6 -> 1.4 + 5.8 ms;
-// 200k x 128, Km = 96: 16 + 12.6 -> 10.2 + 7.8 ms.
+//   * registers held to about 80 (20-24 warps per SM); for rows over 256 floats the query stays in
+//     shared memory.
+// Both rounds on the caller's rows, 1M x 200, Km = 32: 25.5 + 22.5 -> 18.2 + 15.1 ms; 400k x 512,
+// Km = 32: 6.6 + 10.6 -> 1.4 + 5.8 ms; 200k x 128, Km = 96: 16 + 12.6 -> 10.2 + 7.8 ms; 300k x 512,
+// Km = 64: 38 + 59.4 -> 23.3 + 58.5 ms (DRAM-bound; on relocated rows 16.9 + 27.7).
 namespace {
 
 // The query row of the lane's residues, in registers (KSTEPS <= 8) or in shared memory
@@ -117,7 +117,7 @@ struct Query {
 // reference's lane-strided FMA chains), straight from global memory: one warp-wide load reads
 // four 128-byte row segments.  The first log2(R) butterfly levels are transposed (each lane keeps
 // one row), the others plain xor reductions.  Row c0 + 4r + g ends up in lane 8g + m(r).
-template <int KSTEPS, int R>
+template <int KSTEPS, int R, bool FEW>
 __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint32_t d,
                                             const Query<KSTEPS>& q, const uint32_t* list,
                                             uint32_t c0, uint32_t last) {
@@ -131,8 +131,9 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int i = 0; i < 4; i++) p[r][i] = 0.0f;
-  // steps whose loads are in flight together: all of a short row's, else 16 float4 per lane
-  constexpr int KB = KSTEPS > 8 ? 8 / R : R == 4 ? 4 : KSTEPS;
+  // steps whose loads are in flight together: all of them, but half of a long row's when many warps
+  // share the registers
+  constexpr int KB = KSTEPS > 8 && !FEW ? 8 : KSTEPS;
 #pragma unroll
   for (int k0 = 0; k0 < KSTEPS; k0 += KB) {
     float4 x[R][KB];
@@ -200,7 +201,7 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
 }
 
 // Distances of the lanes whose `newc` is set (FLT_MAX elsewhere), up to ROWS rows per pass.
-template <int KSTEPS, int ROWS>
+template <int KSTEPS, int ROWS, bool FEW>
 __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTEPS>& q,
                                            uint32_t node, bool newc, uint32_t* list) {
   const uint32_t lane = lane_id();
@@ -213,15 +214,15 @@ __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTE
   for (uint32_t c0 = 0; c0 < nnew; c0 += ROWS) {
     const uint32_t left = nnew - c0;
     const uint32_t lc = ci - c0, r = lc >> 2;
-    float total;
+    float total = 0.0f;
     uint32_t src = (lc & 3u) << 3;
-    if (left <= 4) {
-      total = score_rows<KSTEPS, 1>(a.base, a.d, q, list, c0, nnew - 1);
-    } else if (ROWS == 8 || left <= 8) {
-      total = score_rows<KSTEPS, 2>(a.base, a.d, q, list, c0, nnew - 1);
+    if (ROWS == 4 || left <= 4) {
+      total = score_rows<KSTEPS, 1, FEW>(a.base, a.d, q, list, c0, nnew - 1);
+    } else if (ROWS <= 8 || left <= 8) {
+      total = score_rows<KSTEPS, 2, FEW>(a.base, a.d, q, list, c0, nnew - 1);
       src |= (r & 1u) << 2;
-    } else {
-      total = score_rows<KSTEPS, 4>(a.base, a.d, q, list, c0, nnew - 1);
+    } else if constexpr (ROWS == 16) {
+      total = score_rows<KSTEPS, 4, FEW>(a.base, a.d, q, list, c0, nnew - 1);
       src |= ((r >> 1) & 1u) << 2 | (r & 1u) << 1;
     }
     const float dd = __shfl_sync(kFull, total, src & 31u);
@@ -233,17 +234,28 @@ __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTE
 
 }  // namespace
 
-// Warps per SM that the registers are allocated for: 23 (Km = 32) and 21 for short rows, 24 for long
-// ones were the fastest of 16..32 (one warp more or less costs 1-3%, 16 or 32 cost 10-30%: too few
-// warps, or spills).
-// Sixteen rows per pass (pg_tuning.search_rows) need 128 registers for their loads.
-constexpr int search_warps(int km_s, int ksteps, int rows) {
-  return rows == 16 ? 16 : ksteps > 8 ? 24 : km_s == 1 ? 23 : 21;
+// Shape by measurement.  Rows per pass: eight short rows (up to 256 floats) whole in flight, four
+// long ones with half of each in flight, or four where eight would spill (short rows past 224
+// floats, Km > 32: 3745 -> 2711 us for 39k queries, Km = 64).  Long rows, eight at a time with a
+// quarter in flight: 4864 queries x 512, Km = 64: 1518 -> 1054 us, and 300k x 512 builds' searches
+// 19.7 + 30.9 -> 16.9 + 27.7 ms.  FEW, for calls with too few queries to fill the SMs, takes the
+// registers that hold 16 short or 8 long rows whole in flight: such a call lasts as long as its
+// longest chain of row reads (608 queries x 512, Km = 64: 601 -> 411 us).
+constexpr int search_rows(int km_s, int ksteps, bool few) {
+  if (few) return ksteps > 8 ? 8 : 16;
+  return ksteps > 8 || (ksteps == 8 && km_s > 1) ? 4 : 8;
 }
 
-template <int KM_S, int KSTEPS, int ROWS>
+// Warps per SM that the registers are allocated for: the fastest of 16..32.  One more or less costs
+// 1-3%, 16 or 32 cost 10-30% (too few warps, or spills).
+constexpr int search_warps(int km_s, int ksteps, bool few) {
+  return few ? 8 : ksteps > 8 ? 24 : km_s == 1 ? 23 : ksteps == 8 ? 20 : 21;
+}
+
+template <int KM_S, int KSTEPS, bool FEW>
 __device__ __forceinline__ void search_queries(const SearchArgs& a) {
   constexpr uint32_t KM = 32u * KM_S;
+  constexpr int ROWS = search_rows(KM_S, KSTEPS, FEW);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t lane = lane_id();
   uint2* merged = reinterpret_cast<uint2*>(smem_raw);                // KM (key, id)
@@ -288,7 +300,7 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
       if (a.place) cand_id = a.place[cand_id];
       // scored for every query at once by k_seed_dists, or here
       const float dist = a.seed_dist ? a.seed_dist[static_cast<uint64_t>(qid) * 32u + lane]
-                                     : score_new<KSTEPS, ROWS>(a, q, cand_id, true, list);
+                                     : score_new<KSTEPS, ROWS, FEW>(a, q, cand_id, true, list);
       cand_key = order_key(dist);
       ev += (lane == 0) ? 32u : 0u;
     }
@@ -345,7 +357,7 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
       const unsigned same = __match_any_sync(kFull, node);
       newc = node != kTomb && (same & lt_mask) == 0 && hash_test_and_set(hash, hmask, node);
       __syncwarp();
-      const float dist = score_new<KSTEPS, ROWS>(a, q, node, newc, list);
+      const float dist = score_new<KSTEPS, ROWS, FEW>(a, q, node, newc, list);
       const unsigned scored = __ballot_sync(kFull, newc);
       ev += (lane == 0) ? __popc(scored) : 0u;
 #pragma unroll
@@ -439,16 +451,15 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
   }
 }
 
-template <int KSTEPS, int ROWS>
-__global__ void __launch_bounds__(32, search_warps(1, KSTEPS, ROWS)) k_search_m32(SearchArgs a) {
-  search_queries<1, KSTEPS, ROWS>(a);
+template <int KSTEPS, bool FEW>
+__global__ void __launch_bounds__(32, search_warps(1, KSTEPS, FEW)) k_search_m32(SearchArgs a) {
+  search_queries<1, KSTEPS, FEW>(a);
 }
 
 // Km = 64, 96
-template <int KM_S, int KSTEPS, int ROWS>
-__global__ void __launch_bounds__(32, search_warps(KM_S, KSTEPS, ROWS))
-    k_search_mk(SearchArgs a) {
-  search_queries<KM_S, KSTEPS, ROWS>(a);
+template <int KM_S, int KSTEPS, bool FEW>
+__global__ void __launch_bounds__(32, search_warps(KM_S, KSTEPS, FEW)) k_search_mk(SearchArgs a) {
+  search_queries<KM_S, KSTEPS, FEW>(a);
 }
 
 // Per warp: the merge buffer, the list of new candidates, the visited set and, for long rows, the
@@ -458,16 +469,16 @@ size_t search_smem(uint32_t km, uint32_t hash_slots, int ksteps, bool qshared) {
          (qshared ? static_cast<size_t>((ksteps + 3) / 4 * 4) * 128 : 0);
 }
 
-template <int KM_S, int KS, int ROWS>
+template <int KM_S, int KS, bool FEW>
 static cudaError_t launch_search_k(const SearchArgs& a, int num_sms, size_t smem_optin,
                                    cudaStream_t st) {
   const size_t smem = search_smem(32u * KM_S, a.hash_slots, KS, kQueryShared<KS>);
   if (smem > smem_optin) return cudaErrorInvalidValue;
   void (*kern)(SearchArgs);
   if constexpr (KM_S == 1)
-    kern = k_search_m32<KS, ROWS>;
+    kern = k_search_m32<KS, FEW>;
   else
-    kern = k_search_mk<KM_S, KS, ROWS>;
+    kern = k_search_mk<KM_S, KS, FEW>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
@@ -741,28 +752,33 @@ bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd) {
          km <= 96 && (km % 32) == 0;
 }
 
+template <int KM_S, int KS>
+static cudaError_t launch_search_few(const SearchArgs& a, bool few, int num_sms,
+                                     size_t smem_optin, cudaStream_t st) {
+  return few ? launch_search_k<KM_S, KS, true>(a, num_sms, smem_optin, st)
+             : launch_search_k<KM_S, KS, false>(a, num_sms, smem_optin, st);
+}
+
+template <int KM_S>
+static cudaError_t launch_search_d(const SearchArgs& a, bool few, int num_sms, size_t smem_optin,
+                                   cudaStream_t st) {
+  if (a.d <= 224) return launch_search_few<KM_S, 7>(a, few, num_sms, smem_optin, st);
+  if (a.d <= 256) return launch_search_few<KM_S, 8>(a, few, num_sms, smem_optin, st);
+  return launch_search_few<KM_S, 16>(a, few, num_sms, smem_optin, st);
+}
+
 cudaError_t launch_search(const SearchArgs& a, int num_sms, size_t smem_optin, cudaStream_t st) {
   if (!search_supported(a.d, a.km, a.kp, a.kd)) return cudaErrorInvalidValue;
   if (a.rows != 0 && a.rows != 8 && a.rows != 16) return cudaErrorInvalidValue;
-  const bool r16 = a.rows == 16;
+  // Few queries: up to eight per SM, one resident round of the FEW kernels.  At sixteen per SM the
+  // others are as fast for long rows and faster for short ones (2432 queries x 200, Km = 32: 136
+  // against 152 us; 1216: 125 against 103).
+  const uint64_t nq = a.queries ? a.nq : a.n;
+  const bool few = nq <= static_cast<uint64_t>(num_sms) * 8 || (a.rows == 16 && a.km == 32);
   switch (a.km / 32) {
-    case 1:
-      if (a.d <= 224)
-        return r16 ? launch_search_k<1, 7, 16>(a, num_sms, smem_optin, st)
-                   : launch_search_k<1, 7, 8>(a, num_sms, smem_optin, st);
-      if (a.d <= 256)
-        return r16 ? launch_search_k<1, 8, 16>(a, num_sms, smem_optin, st)
-                   : launch_search_k<1, 8, 8>(a, num_sms, smem_optin, st);
-      return r16 ? launch_search_k<1, 16, 16>(a, num_sms, smem_optin, st)
-                 : launch_search_k<1, 16, 8>(a, num_sms, smem_optin, st);
-    case 2:
-      if (a.d <= 224) return launch_search_k<2, 7, 8>(a, num_sms, smem_optin, st);
-      return a.d <= 256 ? launch_search_k<2, 8, 8>(a, num_sms, smem_optin, st)
-                        : launch_search_k<2, 16, 8>(a, num_sms, smem_optin, st);
-    default:
-      if (a.d <= 224) return launch_search_k<3, 7, 8>(a, num_sms, smem_optin, st);
-      return a.d <= 256 ? launch_search_k<3, 8, 8>(a, num_sms, smem_optin, st)
-                        : launch_search_k<3, 16, 8>(a, num_sms, smem_optin, st);
+    case 1: return launch_search_d<1>(a, few, num_sms, smem_optin, st);
+    case 2: return launch_search_d<2>(a, few, num_sms, smem_optin, st);
+    default: return launch_search_d<3>(a, few, num_sms, smem_optin, st);
   }
 }
 

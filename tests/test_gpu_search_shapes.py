@@ -1,5 +1,5 @@
 """The beam search at the edges of its kernel shapes -- row lengths around every K-step boundary,
-each beam width, both pass sizes, distances that overflow to infinity -- against the oracle, id for
+each beam width, both pass sizes, few and many queries, distances that overflow to infinity -- against the oracle, id for
 id with equal evaluation and iteration counts."""
 import numpy as np
 import pytest
@@ -34,8 +34,9 @@ def _case(n, d, degree, huge):
 
 @pytest.mark.parametrize("d", [4, 32, 200, 224, 228, 256, 260, 512])
 @pytest.mark.parametrize("km,rows", [(32, 8), (32, 16), (64, 8), (96, 8)])
-def test_search_equals_oracle(pg, d, km, rows):
-    n, degree = 700 + d // 4, 16
+@pytest.mark.parametrize("n", [700, 1500])  # a few queries per SM, and enough to share its registers
+def test_search_equals_oracle(pg, d, km, rows, n):
+    n, degree = n + d // 4, 16
     base, graph = _case(n, d, degree, huge=d in (32, 260))
     ids, ev, it, _ = oracle.search(base, graph, km=km)
     out = torch.full((n, km + 32), -1, dtype=torch.int32, device="cuda")

@@ -71,11 +71,12 @@ size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 struct Layout {
   size_t winner, pruned, pruned_num, indeg, offs, tile_sums, cursor, edges, rev, rev_num, sres,
       proj, graph, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place,
-      pruned_dist, rev_dist, queue, total;
+      pruned_dist, rev_dist, queue, rows16, sdist, total;
 };
 
 Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_t L,
-                   uint32_t proj_deg, uint32_t degree, uint32_t nkeys, uint32_t seg_count = 0) {
+                   uint32_t proj_deg, uint32_t degree, uint32_t nkeys, bool screened,
+                   uint32_t seg_count = 0) {
   Layout l{};
   size_t o = 0;
   auto take = [&](size_t bytes) {
@@ -100,7 +101,11 @@ Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_
   l.proj = take(n * proj_deg * 4);
   l.graph = take(n * degree * 4);
   l.segs = take(2 * (static_cast<size_t>(seg_count) + 1) * 8);
-  l.norms = take(n * 8);  // screened prune: per-point norm bounds
+  if (screened) {  // screened prune: per-point norm bounds, 16-bit rows, the lists' distances
+    l.norms = take(n * 8);
+    l.rows16 = take(n * pg::screen_row(d) * 2);
+    l.sdist = take(n * L * 4);
+  }
   l.seeds = take(n * 32 * 4);  // link-round searches: every query's 32 seed distances
   if (nkeys) {  // relocated build: the sorted copy of the base, seed distances and graphs by place
     l.rbase = take(n * d * 4);
@@ -301,9 +306,11 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   const uint32_t L = p->km + p->kp * p->kd;
   const uint32_t pmax = std::max(p->proj_pruned, p->degree);
   const uint32_t rmax = std::max(p->proj_reverse, p->link_reverse);
+  const bool screened = p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1);
   uint32_t nkeys = p->link_rounds ? pg::reloc_keys(n, d, seg_count) : 0;
   auto shape = [&]() {
-    return make_layout(n, d, pmax, rmax, L, p->proj_degree, p->degree, nkeys, seg_count);
+    return make_layout(n, d, pmax, rmax, L, p->proj_degree, p->degree, nkeys, screened,
+                       seg_count);
   };
   Layout lay = shape();
   if (nkeys && lay.total >= h->reloc_limit) {
@@ -336,11 +343,12 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   uint32_t* proj = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rproj)
                    : proj_out ? proj_out : reinterpret_cast<uint32_t*>(w + lay.proj);
   uint32_t* link = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rgraph) : graph_out;
-  float2* norms = reinterpret_cast<float2*>(w + lay.norms);
+  float2* norms = screened ? reinterpret_cast<float2*>(w + lay.norms) : nullptr;
+  char* rows16 = screened ? w + lay.rows16 : nullptr;
+  uint32_t* sdist = screened ? reinterpret_cast<uint32_t*>(w + lay.sdist) : nullptr;
   float* seeds = reinterpret_cast<float*>(w + lay.seeds);
   uint32_t* order = nkeys ? reinterpret_cast<uint32_t*>(w + lay.order) : nullptr;
   uint32_t* place = nkeys ? reinterpret_cast<uint32_t*>(w + lay.place) : nullptr;
-  const bool screened = p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1);
   unsigned long long* cnt = h->d_counters;
   const int sms = h->num_sms;
   uint64_t* d_seg = nullptr;
@@ -469,6 +477,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.max_iters = p->max_search_iters;
       sa.place = place;
       sa.out = sres;
+      sa.out_key = sdist;
       sa.out_width = L;
       sa.evals = cnt + C_SEARCH + r;
       sa.iters = cnt + C_ITERS + r;
@@ -502,10 +511,14 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       pr.stages = h->tune.screen_stages;
       pr.screen_half = p->screen == PG_SCREEN_FP16;
       pr.norms = norms;
+      pr.rows16 = rows16;
+      pr.cand_dist = reinterpret_cast<const float*>(sdist);
       if (screened) {
         if (r == 0)
-          PG_CUDA(pg::launch_screen_norms(rows, n, d, pr.screen_half, norms, sms, s));
+          PG_CUDA(pg::launch_screen_norms(rows, n, d, pr.screen_half, norms, rows16, sms, s));
+        PG_CUDA(pg::launch_list_dists(rows, n, d, sres, L, sdist, sms, s));
         PG_CUDA(pg::launch_prune_screen(pr, sms, h->smem_optin, s));
+        PG_CUDA(pg::launch_edge_dists(rows, n, d, pruned, pnum, p->degree, pdist, sms, s));
       } else
         PG_CUDA(pg::launch_prune_reverse(pr, false, sms, s));
       PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->degree, n, indeg, offs, tsum, cursor, edges,
@@ -526,7 +539,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       mr.pruned_dist = pdist;
       mr.reverse_dist = rdist;
       mr.own_strict = 1;
-      mr.norms = screened ? norms : nullptr;
+      mr.norms = norms;
       mr.queue = queue;
       mr.degree = p->degree;
       mr.strict = 1;
@@ -900,7 +913,8 @@ int pg_workspace_bytes(const pg_params* p, uint64_t n, uint32_t d, uint64_t q, u
   const uint32_t L = p->km + p->kp * p->kd;
   Layout l = make_layout(n, d, std::max(p->proj_pruned, p->degree),
                          std::max(p->proj_reverse, p->link_reverse), L, p->proj_degree, p->degree,
-                         p->link_rounds ? pg::reloc_keys(n, d, 0) : 0);
+                         p->link_rounds ? pg::reloc_keys(n, d, 0) : 0,
+                         p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1));
   *bytes = l.total;
   return PG_OK;
 }

@@ -81,6 +81,13 @@ __device__ __forceinline__ uint32_t order_key(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// The float of an order_key (+0.0 for both zeros).
+__device__ __forceinline__ float key_dist(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? (key & 0x7FFFFFFFu) : ~key);
+}
+
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;  // a list entry whose distance the search does not know
+
 // (distance, position) -> 64-bit key: sorting these ascending is the stable sort by distance
 // that bubble_sort performs (Gbuilder.cuh:890-902).
 __device__ __forceinline__ uint64_t pack_key(float dist, uint32_t pos) {

@@ -445,6 +445,44 @@ __global__ void __launch_bounds__(32 * W, kPruneWarps / W) k_prune_reverse(Prune
   if (lane_id() == 0 && ev) atomicAdd(a.evals, static_cast<unsigned long long>(ev));
 }
 
+// The distances of the screened prune's kept edges, which the merge sorts by: one edge per lane, the
+// edges of `look` nodes at a time (two or three a node on 1M x 200; at most 32).
+template <bool WIDE>
+__global__ void __launch_bounds__(256) k_edge_dists(const float* __restrict__ base, uint64_t n,
+                                                    uint32_t d,
+                                                    const uint32_t* __restrict__ pruned,
+                                                    const uint32_t* __restrict__ pruned_num,
+                                                    uint32_t p, uint32_t look,
+                                                    float* __restrict__ dist) {
+  const uint32_t lane = lane_id();
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * 8u * look;
+  for (uint64_t b0 = (blockIdx.x * 8ull + (threadIdx.x >> 5)) * look; b0 < n; b0 += stride) {
+    const uint32_t cnt = lane < look && b0 + lane < n ? pruned_num[b0 + lane] : 0u;
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= static_cast<uint32_t>(o)) incl += y;
+    }
+    const uint32_t total = __shfl_sync(kFull, incl, 31);
+    for (uint32_t e0 = 0; e0 < total; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      uint32_t l = 0;  // the number of nodes whose edges all come before e: its node
+#pragma unroll
+      for (uint32_t s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(kFull, incl, l + s - 1) <= e) l += s;
+      const uint32_t before = __shfl_sync(kFull, incl - cnt, l & 31u);
+      if (e < total) {
+        const uint64_t b = b0 + l;
+        const uint64_t at = b * p + (e - before);
+        const uint32_t x = pruned[at];
+        const float v = dist_seq<WIDE>(base + b * d, base + static_cast<uint64_t>(x) * d, d);
+        dist[at] = stored_dist(v, x != static_cast<uint32_t>(b));
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ reverse edges (CSR)
 // Exclusive scan of n counts into offs[0..n] (offs[n] = total).  Three passes: per-block sums,
 // one block scanning the block sums, per-block scan plus offset.
@@ -846,6 +884,17 @@ cudaError_t launch_validate_ids(const uint32_t* ids, uint64_t count, uint64_t n,
 // The 256-bit-load kernels for rows of kWideRowFloats or more on a 32-byte aligned base.
 static bool wide_rows(const float* base, uint32_t d) {
   return d >= kWideRowFloats && (d % 8) == 0 && (reinterpret_cast<uintptr_t>(base) % 32) == 0;
+}
+
+cudaError_t launch_edge_dists(const float* base, uint64_t n, uint32_t d, const uint32_t* pruned,
+                              const uint32_t* pruned_num, uint32_t p, float* dist, int num_sms,
+                              cudaStream_t st) {
+  auto kern = wide_rows(base, d) ? k_edge_dists<true> : k_edge_dists<false>;
+  uint64_t look = n / (static_cast<uint64_t>(num_sms) * 64);  // one round of 64 warps per SM
+  look = look < 1 ? 1 : look > 32 ? 32 : look;
+  kern<<<grid_for(n, static_cast<int>(8 * look), num_sms, 8), 256, 0, st>>>(
+      base, n, d, pruned, pruned_num, p, static_cast<uint32_t>(look), dist);
+  return cudaGetLastError();
 }
 
 template <int W, bool P1>

@@ -35,9 +35,12 @@ struct PruneArgs {
   // depend on it
   uint32_t stages;
   uint32_t screen_half;  // screened kernel: FP16 operands instead of BF16
-  // screened kernel: per point (|x|, |x - x^| + |x^_sub|) upper bounds from launch_screen_norms
-  // with the same screen_half
+  // screened kernel: per point (|x|, |x - x^| + |x^_sub|) upper bounds and the 16-bit rows from
+  // launch_screen_norms with the same screen_half, and the candidates' distances (n x c) from
+  // launch_list_dists
   const float2* norms;
+  const void* rows16;
+  const float* cand_dist;
 };
 
 struct MergeArgs {
@@ -74,6 +77,7 @@ struct SearchArgs {
   uint32_t km, kp, kd, reset_iter, seed_base;
   uint32_t max_iters;
   uint32_t* out;          // n x (km + kp*kd)
+  uint32_t* out_key;      // optional, like out: order_key of the ids' distances (kNoKey: not known)
   unsigned long long* evals;
   unsigned long long* iters;
   uint32_t* work;         // work counter, zeroed before the launch
@@ -244,11 +248,23 @@ bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd);
 // tensor cores + exact re-scoring, 1 <= c <= 128, 4 <= d <= 1024, d % 4 == 0; the launch also
 // wants a 16-byte aligned base.
 bool screen_supported(uint32_t c, uint32_t d, int strict);
+// keys (n x c, c a multiple of 32) of a build's search for lists (n x c) -> the ids' distances to
+// their nodes, in place: the search's, and FP32 inner products where it has none.  FLT_MAX for
+// tombs; the node itself has any value.
+cudaError_t launch_list_dists(const float* base, uint64_t n, uint32_t d, const uint32_t* lists,
+                              uint32_t c, uint32_t* keys, int num_sms, cudaStream_t st);
 cudaError_t launch_prune_screen(const PruneArgs& a, int num_sms, size_t smem_optin,
                                 cudaStream_t st);
-// Per-point norm bounds for the screened prune (FP16 rounding when half, else BF16): n float2.
+// Per-point norm bounds for the screened prune (FP16 rounding when half, else BF16), n float2, and
+// the rounded rows, n x screen_row(d).
 cudaError_t launch_screen_norms(const float* base, uint64_t n, uint32_t d, uint32_t half,
-                                float2* out, int num_sms, cudaStream_t st);
+                                float2* out, void* rows16, int num_sms, cudaStream_t st);
+constexpr uint32_t screen_row(uint32_t d) { return (d + 15u) / 16u * 16u; }
+// The exact chain's distance of every kept edge into dist (n x p), NaN for a node kept in its own
+// list.
+cudaError_t launch_edge_dists(const float* base, uint64_t n, uint32_t d, const uint32_t* pruned,
+                              const uint32_t* pruned_num, uint32_t p, float* dist, int num_sms,
+                              cudaStream_t st);
 
 constexpr uint32_t kScanTileElems = 4096;
 

@@ -2,40 +2,44 @@
 // tensor cores.
 //
 // Same result as k_prune_reverse (strict rounds), bit for bit: the RNG occlusion scan of
-// fusion_prune_reverse_kernel_v0 (Gbuilder.cuh:1093-1244, scan at :1150-1199), each occlusion
-// test dist(p, r) < d_p decided from a screened 16-bit inner product when that lies farther than
-// a proven error bound from d_p, and re-scored with the reference's FP32 chain otherwise.
+// fusion_prune_reverse_kernel_v0 (Gbuilder.cuh:1093-1244, scan at :1150-1199).  Every decision --
+// which candidate is the nearest undecided one, whether dist(p, r) < d_p -- is taken from values
+// whose distance from the reference's FP32 chain is bounded, and from the exact chain where the
+// bound leaves it open.
 //
 // One CTA works on tiles of 128 candidate rows -- two nodes of up to 64 candidates (c <= 64) or
 // one node of up to 128 -- with one thread per tile row (four warps):
-//   1. each warp streams its 32 candidate rows, 32 FP32 columns per chunk, into a ring of S
-//      chunk stages with 16-byte cp.async copies, eight lanes per row segment (coalesced; no
-//      registers held while the copies are in flight; S - 1 chunks run ahead, across tiles),
-//      the 16-byte pieces XOR-swizzled by row so that the 32 threads, one per row, read their
-//      rows without bank conflicts; the node rows come with a tile's first chunk;
-//   2. each thread runs the exact FP32 chain dist(b, x) = -(b . x) of its candidate x against
-//      the node b (distance_between's order, Gbuilder.cuh:785-797) over the chunk, and rounds
-//      the chunk to FP16 (or BF16) into the MMA operand (K-major 8-row x 16-byte core matrices,
-//      no swizzle);
-//   3. one thread issues tcgen05.mma (M = N = 128, K = 16 per instruction, FP32 accumulation)
+//   1. the rows' 16-bit copies (launch_screen_norms) stream into a ring of S chunk stages, 64
+//      columns per chunk, by 16-byte cp.async copies, eight lanes per 128-byte row segment, laid
+//      out as the MMA reads them (128-byte swizzle): the data never pass through registers;
+//   2. one thread issues tcgen05.mma (M = N = 128, K = 16 per instruction, FP32 accumulation)
 //      for the chunk: the Gram G = A A^T of the tile's 16-bit rows accumulates in 128 TMEM
 //      columns, and each node's block of G lies in the node's own TMEM lanes and columns;
-//   4. the node's threads rank their candidates by (exact distance, slot) -- the stable order of
-//      bubble_sort (Gbuilder.cuh:890-902) -- and run the kept-major scan: for each kept entry r
-//      every undecided candidate p reads G[p][r] from its own TMEM lane (one tcgen05.ld column),
-//      decides dist(p, r) < d_p from it outside the bound, or re-scores with the exact chain.
-//      A candidate's recorded occluder is thus the first kept entry, in kept order, that
+//   3. the distance of each candidate to the node comes from the search, which computed it in
+//      another FP32 order (launch_list_dists fills in the few it has not); the nearest undecided candidate is the one whose interval lies below
+//      the others', or the exact minimum (distance, slot) of those whose intervals overlap;
+//   4. for each kept entry r every undecided candidate p reads G[p][r] from its own TMEM lane (one
+//      tcgen05.ld column) and decides dist(p, r) < d_p from it outside the bound, or by exact
+//      chains.  A candidate's recorded occluder is thus the first kept entry, in kept order, that
 //      occludes it, and the kept list equals the reference's one-candidate-at-a-time scan.
-// Error bound (x, y = FP32 rows, x^ = the 16-bit x, e_x = x - x^, Cauchy-Schwarz throughout;
+// Error bounds (x, y = FP32 rows, x^ = the 16-bit x, e_x = x - x^, Cauchy-Schwarz throughout;
 // the two norms per point come from launch_screen_norms, once per build):
 //   |sum x^y^ - sum xy| <= |e_x|(|y| + |e_y|) + |x||e_y|
 //   |MMA(x^, y^) - sum x^y^| <= c_acc (|x| + |e_x|)(|y| + |e_y|)   (FP32 accumulation of Dp terms)
 //   |chain(x, y) - sum xy| <= c_seq |x||y|                          (the reference's FP32 chain)
+//   |search(x, y) - sum xy| <= c_par |x||y|                         (the search's FP32 order)
 // with c_acc = (Dp + 32) 2^-21 (eight times the sequential-summation bound, covering the tensor
-// core's accumulation) and c_seq = (D + 2) 2^-23, plus a 2^-20 relative guard on the comparison.
+// core's accumulation), c_seq = (D + 2) 2^-23 and c_par = (D / 32 + 10) 2^-23 (the search's
+// D / 32 + 6 roundings of 2^-24), plus a 2^-20 relative guard on each comparison.
 // Values beyond FP16's range give infinite norms, which send every test of that node to the
 // exact chain.  Every mbarrier wait is bounded (one second); a thread that gives up makes the
 // whole CTA stop at its next barrier and raises kErrWait.
+// Bound by the latency of a tile's steps (copies, MMAs, then two exchanges per kept entry) and the
+// L2 gathers.  Streaming the FP32 rows instead, with the exact chain and the rounding of every
+// candidate done by its thread, and exact chains for every test inside the 16-bit margin, took
+// 10.6 + 10.7 ms at 1M x 200 and 22 + 31 ms at 300k x 512, L = 96.  Now 7.1 + 7.6 ms, with 0.5 ms
+// each for launch_list_dists and launch_edge_dists, and 17 + 29 ms with them.  Two or four stages
+// are 2-4% slower than three.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -52,63 +56,37 @@ using namespace tcu;
 
 constexpr uint32_t kTile = 128;                 // tile rows = MMA M = N = TMEM columns = threads
 constexpr uint32_t kWarps = kTile / 32;
-constexpr uint32_t kCk = 32;                    // FP32 columns per chunk
-constexpr uint32_t kRowBytes = kCk * 4;         // bytes per row and chunk (eight 16-byte pieces)
-constexpr uint32_t kStageBytes = kTile * kRowBytes;
-constexpr uint32_t kOpBytes = kTile * kCk * 2;  // one 16-bit chunk of the tile
-constexpr uint32_t kLbo = 128;                  // core matrices along K
-constexpr uint32_t kSbo = 512;                  // core matrices along M / N (8-row groups)
+constexpr uint32_t kCk = 64;                    // 16-bit columns per chunk: 128 bytes of a row
+constexpr uint32_t kStageBytes = kTile * 128;
 constexpr uint32_t kBarAll = 1, kBarNode = 2;   // named barriers: all threads; node 0 (+ node)
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 struct TcShape {
   uint32_t cap;    // candidate slots per node: 64 (two nodes per tile) or 128 (one)
+  uint32_t dp;     // 16-bit row length: D rounded up to 16
   uint32_t nk;     // chunks per row
-  uint32_t nbuf;   // node-row buffers (tiles whose node rows are in flight or in use)
-  uint32_t dpad;   // floats per staged node row: D rounded up to the chunk
   uint64_t tiles;  // ceil(n / nodes per tile)
 };
 
 // Shared-memory layout, offsets from a 1024-byte aligned base.
 struct Layout {
-  uint32_t op, stage, nrow, key, id, nrm, err, xch, bars, words, total;
+  uint32_t stage, id, nrm, err, last, xch, bars, words, total;
 };
-__host__ __device__ constexpr Layout layout(uint32_t stages, uint32_t nbuf, uint32_t dpad) {
+__host__ __device__ constexpr Layout layout(uint32_t stages) {
   Layout l{};
-  l.op = 0;
-  l.stage = l.op + 2 * kOpBytes;
-  l.nrow = l.stage + stages * kStageBytes;
-  l.key = l.nrow + nbuf * 2 * dpad * 4;  // multiple of 16
-  l.id = l.key + kTile * 8;
+  l.stage = 0;
+  l.id = stages * kStageBytes;
   l.nrm = l.id + kTile * 4;
   l.err = l.nrm + kTile * 4;
-  l.xch = l.err + kTile * 4;
-  l.bars = l.xch + 2 * kWarps * 4;  // opfree[2], acc, drained
-  l.words = l.bars + 4 * 8;         // TMEM address
+  l.last = l.err + kTile * 4;       // per node: the last kept entry's distance and bound
+  l.xch = l.last + 2 * 8;
+  l.bars = l.xch + 2 * kWarps * 4;  // free[stages], acc, drained
+  l.words = l.bars + (stages + 2) * 8;  // TMEM address
   l.total = l.words + 16;
   return l;
 }
-// Stages of the copy ring (chunks in flight per thread + the one consumed); the default can be
-// set at build time with -DPG_PRUNE_TC_STAGES.
-#ifndef PG_PRUNE_TC_STAGES
-#define PG_PRUNE_TC_STAGES 2
-#endif
-constexpr uint32_t kMinStages = 2, kMaxStages = 4, kDefaultStages = PG_PRUNE_TC_STAGES;
-size_t smem_bytes(uint32_t stages, const TcShape& sh) {
-  return layout(stages, sh.nbuf, sh.dpad).total + 1024;
-}
-
-// Two floats rounded to the screening type (FP16 when HALF, else BF16), packed.
-template <bool HALF>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (HALF) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-  } else {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
-  }
-}
+constexpr uint32_t kMinStages = 2, kMaxStages = 4, kDefaultStages = 3;
+size_t smem_bytes(uint32_t stages) { return layout(stages).total + 1024; }
 
 // 16 bytes global -> shared, cached in L2 only, completing with the thread's copy groups.
 __device__ __forceinline__ void cp16(void* dst, const void* src) {
@@ -155,21 +133,43 @@ __device__ __forceinline__ bool named_and(uint32_t id, uint32_t threads, bool v)
   return r != 0;
 }
 
-// Minimum of v over the threads of one node (warps col0 / 32 .. + nw - 1, named barrier
-// bar_node); every thread of the node makes the same sequence of calls, numbered by q.
-__device__ __forceinline__ uint32_t node_min(uint32_t v, uint32_t* xch, uint32_t& q,
-                                             uint32_t col0, uint32_t nw, uint32_t bar_node,
-                                             uint32_t threads) {
-  v = __reduce_min_sync(kFull, v);
-  uint32_t* xb = xch + (q & 1u) * kWarps;
-  if ((threadIdx.x & 31u) == 0) xb[threadIdx.x >> 5] = v;
-  __syncwarp();
-  named_sync(bar_node, threads);
-  uint32_t m = kNone;
-  for (uint32_t w = 0; w < nw; w++) m = min(m, xb[col0 / 32u + w]);
-  q++;
-  return m;
-}
+// The threads of one node: warps col0 / 32 .. + nw - 1, named barrier `bar`.  Every thread of the
+// node makes the same sequence of exchanges, numbered by q.
+struct Node {
+  uint32_t* xch;
+  uint32_t w0, nw, bar, threads;
+  uint32_t q;
+  // One word per warp of the node, seen by all its threads.
+  __device__ __forceinline__ const uint32_t* exchange(uint32_t v) {
+    uint32_t* xb = xch + (q & 1u) * kWarps;
+    q++;
+    if ((threadIdx.x & 31u) == 0) xb[threadIdx.x >> 5] = v;
+    __syncwarp();
+    named_sync(bar, threads);
+    return xb + w0;
+  }
+  __device__ __forceinline__ uint32_t min(uint32_t v) {
+    const uint32_t* x = exchange(__reduce_min_sync(kFull, v));
+    uint32_t m = kNone;
+    for (uint32_t w = 0; w < nw; w++) m = ::min(m, x[w]);
+    return m;
+  }
+  // How many threads hold f, and the lowest slot that does (kNone: none).
+  __device__ __forceinline__ uint32_t count(bool f, uint32_t& first) {
+    const uint32_t* x = exchange(__ballot_sync(kFull, f));
+    uint32_t c = 0;
+    first = kNone;
+    for (uint32_t w = 0; w < nw; w++) {
+      const uint32_t m = x[w];
+      if (m && first == kNone) first = 32u * w + static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
+      c += __popc(m);
+    }
+    return c;
+  }
+};
+
+// order_key with the largest value left free to mean "none".
+__device__ __forceinline__ uint32_t dist_key(float f) { return min(order_key(f), kNone - 1u); }
 
 // This thread's candidate id in tile t, or kNone when the slot holds no row to stage (past the
 // end, a tomb, an out-of-range id or the node itself).
@@ -181,81 +181,154 @@ __device__ __forceinline__ uint32_t cand_id(const PruneArgs& a, uint64_t t, uint
   return (x >= a.n || x == static_cast<uint32_t>(b)) ? kNone : x;
 }
 
-// The copy stream of one thread: the chunks of its warp's rows in the CTA's tile order, S - 1
-// chunks ahead of the one being consumed, one cp.async group per chunk (empty past the last
-// tile).
+// The copy stream of one thread: the chunks of its warp's rows in the CTA's tile order, one
+// cp.async group per chunk (empty past the last tile).
 struct Feed {
-  uint64_t t;  // tile of the next chunk to issue
+  uint64_t t;   // tile of the next chunk to issue
   uint32_t kc;  // the chunk
-  uint32_t lt;  // the tile's index among this CTA's tiles (selects the node-row buffer)
   uint32_t x;   // this thread's candidate id in tile t (kNone: nothing to stage)
 };
 
-// Issues chunk f.kc of tile f.t into stage gi % S.  The warp copies its 32 rows four at a time:
-// eight lanes per row, one 16-byte piece each, so that each copy instruction reads whole row
-// segments (coalesced) rather than one piece of 32 rows.
-template <uint32_t S>
+// Issues chunk f.kc of tile f.t into `st`.  The warp copies its 32 rows four at a time: eight lanes
+// per row, one 16-byte piece each, so that each copy instruction reads whole row segments, swizzled
+// as the MMA's descriptors expect (piece j of row r at j ^ (r mod 8) of its 128 bytes).
 __device__ __forceinline__ void feed_issue(Feed& f, const PruneArgs& a, const TcShape& sh,
-                                           uint8_t* stage, float* nrow, uint32_t gi, uint32_t P,
-                                           uint32_t node, uint32_t slot) {
+                                           uint8_t* st, uint32_t P, uint32_t node, uint32_t slot) {
   const uint32_t R = threadIdx.x, lane = R & 31u;
   if (f.t < sh.tiles) {
-    const uint32_t pieces = min(kCk, a.d - f.kc * kCk) / 4;
+    const uint32_t pieces = min(kCk, sh.dp - f.kc * kCk) / 8;
     const uint32_t j = lane & 7u;
-    uint8_t* st = stage + (gi % S) * kStageBytes;
+    const uint8_t* src = static_cast<const uint8_t*>(a.rows16) + f.kc * 128u + 16u * j;
 #pragma unroll
     for (uint32_t i = 0; i < 8; i++) {
       const uint32_t rr = (R & ~31u) + 4u * i + (lane >> 3);  // tile row copied by this lane
       const uint32_t xr = __shfl_sync(kFull, f.x, 4u * i + (lane >> 3));
       if (xr != kNone && j < pieces)
-        cp16(st + rr * kRowBytes + ((j ^ (rr & 7u)) << 4),
-             reinterpret_cast<const char*>(a.base + static_cast<uint64_t>(xr) * a.d) +
-                 f.kc * kRowBytes + 16u * j);
-    }
-    if (f.kc == 0) {  // the node rows of the tile, 16-byte pieces spread over the node's threads
-      const uint64_t b = f.t * P + node;
-      if (b < a.n) {
-        const char* nsrc = reinterpret_cast<const char*>(a.base + b * a.d);
-        float* nb = nrow + ((f.lt % sh.nbuf) * 2 + node) * sh.dpad;
-        for (uint32_t i = slot; i < a.d / 4; i += sh.cap) cp16(nb + 4 * i, nsrc + 16u * i);
-      }
+        cp16(st + rr * 128u + ((j ^ (rr & 7u)) << 4), src + static_cast<uint64_t>(xr) * (2u * sh.dp));
     }
     if (++f.kc == sh.nk) {
       f.kc = 0;
       f.t += gridDim.x;
-      f.lt++;
       f.x = f.t < sh.tiles ? cand_id(a, f.t, P, node, slot) : kNone;
     }
   }
   cp_commit();
 }
 
+// FP32 inner products of row r with the rows x of the lanes that `want` one, each valid in its lane:
+// four at a time, eight lanes per row, so that the loads are whole 128-byte lines.
+__device__ __forceinline__ float warp_dots(const float* __restrict__ base, uint32_t d, uint32_t r,
+                                           uint32_t x, bool want) {
+  const uint32_t lane = threadIdx.x & 31u, g = lane >> 3, m = lane & 7u;
+  unsigned todo = __ballot_sync(kFull, want);
+  const float* rrow = base + static_cast<uint64_t>(r) * d;
+  float mine = 0.f;
+  while (todo) {
+    unsigned t = todo;
+    for (uint32_t i = 0; i < g; i++) t &= t - 1u;  // group g takes the g-th lane, or repeats one
+    const int src = __ffs(static_cast<int>(t ? t : todo)) - 1;
+    const float* xrow = base + static_cast<uint64_t>(__shfl_sync(kFull, x, src)) * d;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (uint32_t c = 4u * m; c < d; c += 32) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(rrow + c));
+      const float4 v = __ldg(reinterpret_cast<const float4*>(xrow + c));
+      s.x = fmaf(u.x, v.x, s.x);
+      s.y = fmaf(u.y, v.y, s.y);
+      s.z = fmaf(u.z, v.z, s.z);
+      s.w = fmaf(u.w, v.w, s.w);
+    }
+    float v = (s.x + s.y) + (s.z + s.w);
+    v += __shfl_xor_sync(kFull, v, 4);
+    v += __shfl_xor_sync(kFull, v, 2);
+    v += __shfl_xor_sync(kFull, v, 1);
+    const uint32_t rank = __popc(todo & ((1u << lane) - 1u));
+    const float got = __shfl_sync(kFull, v, static_cast<int>((rank & 3u) << 3));
+    if (((todo >> lane) & 1u) && rank < 4) mine = got;
+    for (uint32_t i = 0; i < 4; i++) todo &= todo - 1u;  // 0 stays 0
+  }
+  return mine;
+}
+
+// One warp per list of 32 E entries: the distances that its search does not know belong to ids that
+// it had visited before its last step.  Such an id may stand elsewhere in the list; the others are
+// scored.
+template <int E>
+__global__ void __launch_bounds__(256) k_list_dists(const float* __restrict__ base, uint64_t n,
+                                                    uint32_t d, const uint32_t* __restrict__ lists,
+                                                    uint32_t* __restrict__ keys) {
+  constexpr uint32_t C = 32u * E;
+  __shared__ uint4 ids_all[8][C / 4];
+  __shared__ uint32_t key_all[8][C];
+  uint4* ids = ids_all[threadIdx.x >> 5];
+  uint32_t* ks = key_all[threadIdx.x >> 5];
+  const uint32_t lane = lane_id();
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * 8;
+  for (uint64_t b = blockIdx.x * 8ull + (threadIdx.x >> 5); b < n; b += nw) {
+    uint32_t id[E], key[E];
+    bool any = false;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      id[e] = lists[b * C + 32 * e + lane];
+      key[e] = keys[b * C + 32 * e + lane];
+      if (id[e] >= n) key[e] = order_key(FLT_MAX);
+      if (key[e] == kNoKey && id[e] == static_cast<uint32_t>(b)) key[e] = order_key(FLT_MAX);
+      any |= key[e] == kNoKey;
+    }
+    if (__any_sync(kFull, any)) {
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        reinterpret_cast<uint32_t*>(ids)[32 * e + lane] = id[e];
+        ks[32 * e + lane] = key[e];
+      }
+      __syncwarp();
+#pragma unroll
+      for (int e = 0; e < E; e++) {
+        if (!__any_sync(kFull, key[e] == kNoKey)) continue;
+        uint32_t at = 32u * e + lane;  // another entry of the same id whose distance is known
+#pragma unroll 4
+        for (uint32_t j = 0; j < C / 4; j++) {
+          const uint4 v = ids[j];
+          if (v.x == id[e] && ks[4 * j] != kNoKey) at = 4 * j;
+          if (v.y == id[e] && ks[4 * j + 1] != kNoKey) at = 4 * j + 1;
+          if (v.z == id[e] && ks[4 * j + 2] != kNoKey) at = 4 * j + 2;
+          if (v.w == id[e] && ks[4 * j + 3] != kNoKey) at = 4 * j + 3;
+        }
+        if (key[e] == kNoKey) key[e] = ks[at];
+        const bool want = key[e] == kNoKey;
+        const float s32 = warp_dots(base, d, static_cast<uint32_t>(b), id[e], want);
+        if (want) key[e] = order_key(-s32);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++) keys[b * C + 32 * e + lane] = __float_as_uint(key_dist(key[e]));
+    __syncwarp();
+  }
+}
+
 template <bool HALF, uint32_t S>
-__global__ void __launch_bounds__(kTile, S == 2 ? 4 : 3) k_prune_tc(const PruneArgs a, const TcShape sh) {
+__global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneArgs a,
+                                                                   const TcShape sh) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   uint8_t* sm = smem_raw + ((1024u - (saddr(smem_raw) & 1023u)) & 1023u);
-  const Layout L = layout(S, sh.nbuf, sh.dpad);
-  uint8_t* op = sm + L.op;
+  constexpr Layout L = layout(S);
   uint8_t* stage = sm + L.stage;
-  float* nrow = reinterpret_cast<float*>(sm + L.nrow);
-  uint64_t* skey = reinterpret_cast<uint64_t*>(sm + L.key);
   uint32_t* sid = reinterpret_cast<uint32_t*>(sm + L.id);
   float* snrm = reinterpret_cast<float*>(sm + L.nrm);
   float* serr = reinterpret_cast<float*>(sm + L.err);
-  uint32_t* xch = reinterpret_cast<uint32_t*>(sm + L.xch);
-  uint64_t* opfree = reinterpret_cast<uint64_t*>(sm + L.bars);  // [2]
-  uint64_t* accfull = opfree + 2;
+  float2* slast = reinterpret_cast<float2*>(sm + L.last);
+  uint64_t* sfree = reinterpret_cast<uint64_t*>(sm + L.bars);  // [S]
+  uint64_t* accfull = sfree + S;
   uint64_t* drained = accfull + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + L.words);
 
   const uint32_t R = threadIdx.x, warp = R >> 5, lane = R & 31u;
   const uint32_t cap = sh.cap, P = kTile / cap;
   const uint32_t node = R / cap, slot = R - node * cap, col0 = node * cap;
-  const uint32_t bar_node = kBarNode + node, nw = cap / 32u;
+  Node nd{reinterpret_cast<uint32_t*>(sm + L.xch), col0 / 32u, cap / 32u, kBarNode + node, cap, 0};
 
   if (R == 0) {
-    bar_init(opfree, 1);
-    bar_init(opfree + 1, 1);
+    for (uint32_t i = 0; i < S; i++) bar_init(sfree + i, 1);
     bar_init(accfull, 1);
     bar_init(drained, 1);
     fence_barrier_init();
@@ -268,159 +341,198 @@ __global__ void __launch_bounds__(kTile, S == 2 ? 4 : 3) k_prune_tc(const PruneA
   const uint32_t taddr = tmem + ((warp * 32u) << 16);
 
   const uint32_t d = a.d;
-  const float c_acc = static_cast<float>((d + 15u) / 16u * 16u + 32u) * 4.76837158e-07f;  // 2^-21
-  const float c_seq = static_cast<float>(d + 2u) * 1.19209290e-07f;                   // 2^-23
+  const float c_acc = static_cast<float>(sh.dp + 32u) * 4.76837158e-07f;  // 2^-21
+  const float c_seq = static_cast<float>(d + 2u) * 1.19209290e-07f;       // 2^-23
+  const float c_par = static_cast<float>(d / 32u + 10u) * 1.19209290e-07f;
+  constexpr float kGuard = 9.5367431640625e-07f;                         // 2^-20
+  const uint32_t kmax = order_key(FLT_MAX);
   // A and B FP16 (format 0) or BF16 (format 1, bits 7-9 and 10-12)
   constexpr uint32_t kIdesc = idesc_f16(kTile, kTile) | (HALF ? 0u : ((1u << 7) | (1u << 10)));
   uint64_t ev = 0, resc = 0;
-  uint32_t g = 0, q = 0, it = 0;
-  bool ok = true;
+  uint32_t g = 0, it = 0;
+  bool ok = true, w = true;
 
-  Feed f{blockIdx.x, 0, 0, kNone};
+  Feed f{blockIdx.x, 0, kNone};
   if (f.t < sh.tiles) f.x = cand_id(a, f.t, P, node, slot);
-  for (uint32_t i = 0; i + 1 < S; i++) feed_issue<S>(f, a, sh, stage, nrow, i, P, node, slot);
+  for (uint32_t i = 0; i + 1 < S; i++)
+    feed_issue(f, a, sh, stage + i * kStageBytes, P, node, slot);
+  // the scan's inputs are read a tile ahead: ids and distances, then the norms that hang on them
+  uint32_t x_next = kTomb;
+  float dist_next = FLT_MAX;
+  auto fetch = [&](uint64_t t) {
+    const uint64_t b = t * P + node;
+    const bool in = t < sh.tiles && b < a.n && slot < a.c;
+    x_next = in ? a.graph[b * a.c + slot] : kTomb;
+    dist_next = in ? a.cand_dist[b * a.c + slot] : FLT_MAX;
+  };
+  fetch(blockIdx.x);
 
   for (uint64_t t = blockIdx.x; t < sh.tiles; t += gridDim.x, it++) {
     const uint64_t b = t * P + node;
     const bool bval = b < a.n;
-    uint32_t x = kTomb;
-    if (bval && slot < a.c) {
-      x = a.graph[b * a.c + slot];
-      if (x >= a.n && x != kTomb && x != kMaskedTomb) {
-        raise_error(a.status, kErrBadId);
-        x = kTomb;
-      }
+    uint32_t x = x_next;
+    float dist = dist_next;  // of the candidate to the node: within `bound` of the exact chain's
+    if (x >= a.n && x != kTomb && x != kMaskedTomb) {
+      raise_error(a.status, kErrBadId);
+      x = kTomb;
     }
-    const bool valid = bval && x != kTomb && x != kMaskedTomb && x != static_cast<uint32_t>(b);
-    const float* nb = nrow + ((it % sh.nbuf) * 2 + node) * sh.dpad;
-    float acc = 0.f;
+    const bool in = bval && slot < a.c;
+    const bool tomb = in && (x == kTomb || x == kMaskedTomb);
+    const bool valid = in && !tomb && x != static_cast<uint32_t>(b);
+    const float2 ne = valid ? __ldg(a.norms + x) : make_float2(0.f, 0.f);
+    const float nb = bval ? __ldg(&a.norms[b].x) : 0.f;
+    fetch(t + gridDim.x);
     for (uint32_t kc = 0; kc < sh.nk; kc++, g++) {
-      feed_issue<S>(f, a, sh, stage, nrow, g + S - 1, P, node, slot);
-      cp_wait<S - 1>();  // this thread's copies of chunk g have landed; after the warp
-      __syncwarp();      // barrier, so have the copies of this thread's row by the others
-      if (kc == 0) named_sync(kBarAll, kTile);  // and the node-row pieces, for a first chunk
-      const uint32_t kn = min(kCk, d - kc * kCk);  // columns in this chunk, a multiple of 4
-      const uint8_t* rp = stage + (g % S) * kStageBytes + R * kRowBytes;
-      const float* np = nb + kc * kCk;
-      uint32_t h[16];
-#pragma unroll
-      for (uint32_t j = 0; j < 8; j++) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (valid && 4u * j < kn) {
-          v = *reinterpret_cast<const float4*>(rp + ((j ^ (R & 7u)) << 4));
-          const float4 u = *reinterpret_cast<const float4*>(np + 4u * j);
-          acc = fmaf(u.x, v.x, acc);
-          acc = fmaf(u.y, v.y, acc);
-          acc = fmaf(u.z, v.z, acc);
-          acc = fmaf(u.w, v.w, acc);
-        }
-        h[2 * j] = pack2<HALF>(v.x, v.y);
-        h[2 * j + 1] = pack2<HALF>(v.z, v.w);
-      }
-      const uint32_t o = g & 1u;
-      bool w = true;
-      if (g >= 2) w = bar_wait_hint(opfree + o, ((g >> 1) + 1u) & 1u);  // MMAs of chunk g - 2
-      if (w) {
-        uint8_t* dst = op + o * kOpBytes + (R >> 3) * kSbo + (R & 7u) * 16u;
-#pragma unroll
-        for (uint32_t j = 0; j < 4; j++)
-          *reinterpret_cast<uint4*>(dst + j * kLbo) =
-              make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
-      }
+      cp_wait<S - 2>();  // this thread's copies of chunk g have landed
       fence_proxy_async();
-      __syncwarp();
-      ok = named_and(kBarAll, kTile, w);
+      ok = named_and(kBarAll, kTile, w);  // and everyone's
       if (!ok) break;
       if (R == 0) {
         fence_after();
-        const uint32_t a0 = saddr(op + o * kOpBytes);
-        const uint32_t steps = (kn + 15u) >> 4;
+        const uint32_t a0 = saddr(stage + (g % S) * kStageBytes);
+        const uint32_t steps = min(kCk, sh.dp - kc * kCk) / 16u;
         for (uint32_t k = 0; k < steps; k++) {
-          const uint64_t dsc = plain_desc(a0 + k * 2u * kLbo, kLbo, kSbo);
+          const uint64_t dsc = sw128_desc(a0 + 32u * k);
           mma_f16(tmem, dsc, dsc, kIdesc, (kc | k) != 0);
         }
-        commit(opfree + o);  // the operand buffer is free once these MMAs have read it
+        commit(sfree + g % S);  // the stage is free once these MMAs have read it
         if (kc + 1 == sh.nk) commit(accfull);
       }
+      // the next chunk of the stream goes where chunk g - 1 was
+      const uint32_t at = (g + S - 1) % S;
+      if (g >= 1) w = __all_sync(kFull, bar_wait_hint(sfree + at, ((g - 1) / S) & 1u));
+      if (w)
+        feed_issue(f, a, sh, stage + at * kStageBytes, P, node, slot);
+      else
+        cp_commit();
     }
     if (!ok) break;
+    sid[R] = x;
+    snrm[R] = ne.x;
+    serr[R] = ne.y;
     __syncwarp();
-    ok = named_and(kBarAll, kTile, bar_wait_hint(accfull, it & 1u));
+    ok = named_and(kBarAll, kTile, w && bar_wait_hint(accfull, it & 1u));
     if (!ok) break;
     fence_after();
 
     // ---- the node's scan
-    const bool in = slot < a.c;
-    const float dist = valid ? -acc : FLT_MAX;
-    const float2 ne = valid ? __ldg(a.norms + x) : make_float2(0.f, 0.f);
-    skey[R] = in ? pack_key(dist, slot) : ~0ull;
-    sid[R] = x;
-    snrm[R] = ne.x;
-    serr[R] = ne.y;
+    const float* brow = a.base + (bval ? b : 0) * d;
+    const float* xrow = a.base + static_cast<uint64_t>(valid ? x : 0u) * d;
+    float bound = 0.f;  // 0: dist is the exact chain's (or FLT_MAX)
+    auto exact = [&]() {  // a settlement holds up the scan: 256-bit loads whatever the row length
+      dist = dist_seq<true>(brow, xrow, d);
+      bound = 0.f;
+    };
+    if (valid) {
+      bound = 0.5f * (c_seq + c_par) * nb * ne.x + fabsf(dist) * 2.4e-7f + 1e-30f;
+      if (!(fabsf(dist) < 1e37f && bound < 1e37f)) exact();
+    } else {
+      dist = FLT_MAX;
+    }
     const uint32_t nv = __popc(__ballot_sync(kFull, valid));
     if (lane == 0) ev += nv;
-    __syncwarp();
-    named_sync(bar_node, cap);
-    uint32_t pos = kNone;
-    if (in) {
-      const uint64_t my = skey[R];
-      uint32_t r = 0;
-      for (uint32_t j = 0; j < a.c; j++) r += skey[col0 + j] < my ? 1u : 0u;
-      pos = r;
+    // undecided: candidates that come before the first tomb in (distance, slot) order
+    uint32_t first_tomb;
+    const uint32_t tombs = nd.count(tomb, first_tomb);
+    bool open = in && !tomb;
+    if (open && tombs) {
+      const uint32_t key = dist_key(dist);
+      open = key < kmax || (key == kmax && slot < first_tomb);
     }
-    const bool tomb = in && (x == kTomb || x == kMaskedTomb);
-    // the first tomb in sorted order, and the slot at sorted position 0
-    const uint32_t tend = node_min(tomb ? pos : a.c, xch, q, col0, nw, bar_node, cap);
-    const uint32_t k0 = node_min(in ? (pos << 8) | slot : kNone, xch, q, col0, nw, bar_node, cap);
-    uint32_t K = 0, my_kept = kNone;
-    if (tend != 0 && k0 != kNone) {
-      K = 1;
-      uint32_t ro = k0 & 0xFFu, last = 0, jend = 1, nres = 0, fo = kNone;
-      if (slot == ro) my_kept = 0;
-      while (a.p > 1) {
-        const uint32_t t_k = K - 1;
-        const uint32_t ri = sid[col0 + ro];
-        const float nr = snrm[col0 + ro], er = serr[col0 + ro];
-        const float gv = __uint_as_float(tmem_ld1(taddr + col0 + ro));
-        tmem_wait_ld();
-        if (in && pos > last && pos < tend && fo == kNone) {
+    // The undecided candidate that comes first: the one whose interval may hold the smallest
+    // distance, or, among several, the exact minimum.
+    auto next = [&]() -> uint32_t {
+      for (uint32_t pass = 0;; pass++) {
+        const uint32_t m = nd.min(open ? dist_key(dist + bound) : kNone);
+        if (m == kNone) return kNone;
+        const bool may = open && dist_key(dist - bound) <= m;
+        uint32_t s;
+        if (nd.count(may, s) == 1 || pass) return s;
+        if (may && bound > 0.f) exact();
+      }
+    };
+    uint32_t K = 0, my_kept = kNone, fo = kNone;
+    bool full = false;
+    uint32_t ro = next();
+    while (ro != kNone) {
+      if (slot == ro) {
+        my_kept = K;
+        open = false;
+      }
+      const uint32_t t_k = K++;
+      if (K == a.p) {
+        full = true;
+        break;
+      }
+      const uint32_t ri = sid[col0 + ro];
+      const float nr = snrm[col0 + ro], er = serr[col0 + ro];
+      const float gv = __uint_as_float(tmem_ld1(taddr + col0 + ro));
+      tmem_wait_ld();
+      bool yes = false, sure = !open;
+      const bool other = ri != static_cast<uint32_t>(b);  // the node itself has no row in the tile
+      if (open && other) {
+        if (valid) {
           const float dhat = -gv;
-          const float np2 = ne.x, ep = ne.y;
-          const float bound = ep * (nr + er) + np2 * er + c_acc * (np2 + ep) * (nr + er) +
-                              c_seq * np2 * nr + fabsf(dhat) * 9.5367431640625e-07f + 1e-30f;
-          bool yes = dhat + bound < dist;
-          if (!yes && !(dhat - bound >= dist)) {  // inside the margin (or NaN): exact chain
-            // a re-score holds up the node's scan: 256-bit loads whatever the row length
+          const float e = ne.y * (nr + er) + ne.x * er + c_acc * (ne.x + ne.y) * (nr + er) +
+                          c_seq * ne.x * nr + fabsf(dhat) * kGuard + 1e-30f + bound;
+          yes = dhat + e < dist;
+          sure = yes || dhat - e >= dist;
+        } else if (nb * nr < 1e37f) {  // the node: at FLT_MAX, past any chain this bounds
+          yes = sure = true;
+        }
+      }
+      const uint32_t nun = __popc(__ballot_sync(kFull, !sure));
+      if (nun) {  // inside the 16-bit margin: FP32 products, exact chains inside theirs (or NaN)
+        const float s32 = warp_dots(a.base, d, ri, x, !sure && valid && other);
+        if (!sure) {
+          if (valid && other) {
+            const float dhat = -s32;
+            const float e = (c_seq + c_par) * ne.x * nr + fabsf(dhat) * kGuard + 1e-30f + bound;
+            yes = dhat + e < dist;
+            sure = yes || dhat - e >= dist;
+          }
+          if (!sure) {
+            if (bound > 0.f) exact();
             yes = dist_seq<true>(a.base + static_cast<uint64_t>(x) * d,
                                  a.base + static_cast<uint64_t>(ri) * d, d) < dist;
-            nres++;
           }
-          if (yes) fo = t_k;
         }
-        const uint32_t nk = node_min(
-            (in && pos > last && pos < tend && fo == kNone) ? (pos << 8) | slot : kNone, xch, q,
-            col0, nw, bar_node, cap);
-        if (nk == kNone) {  // no undecided candidate before the first tomb
-          jend = tend;
-          break;
-        }
-        ro = nk & 0xFFu;
-        if (slot == ro) my_kept = K;
-        K++;
-        last = nk >> 8;
-        if (K == a.p) {
-          jend = last + 1;
-          break;
-        }
+        if (lane == 0) resc += nun;
       }
-      const uint32_t ch = (in && pos >= 1 && pos < jend && fo != kNone) ? fo + 1 : 0u;
-      const uint32_t chs = __reduce_add_sync(kFull, ch);
-      const uint32_t rs = __reduce_add_sync(kFull, nres);
-      if (lane == 0) {
-        ev += chs;
-        resc += rs;
+      if (open && yes) {
+        fo = t_k;
+        open = false;
       }
+      ro = next();
     }
+    // evaluations: the occluded candidates that come before the entry that filled the list
+    bool counted = fo != kNone;
+    if (full) {
+      auto tell = [&]() {
+        if (my_kept == K - 1) slast[node] = make_float2(dist, bound);
+        __syncwarp();
+        named_sync(nd.bar, nd.threads);
+        return slast[node];
+      };
+      float2 l = tell();
+      bool unsure = counted && !(dist_key(dist + bound) < dist_key(l.x - l.y)) &&
+                    !(dist_key(dist - bound) > dist_key(l.x + l.y));
+      uint32_t s;
+      if (nd.count(unsure, s)) {  // also separates the two uses of slast
+        if ((unsure || my_kept == K - 1) && bound > 0.f) exact();
+        l = tell();
+      }
+      if (counted) {
+        const uint32_t key = dist_key(dist - bound), lkey = dist_key(l.x + l.y);
+        counted = unsure ? dist_key(dist) < dist_key(l.x) ||
+                               (dist_key(dist) == dist_key(l.x) && slot < ro)
+                         : !(key > lkey);
+      }
+      __syncwarp();
+      named_sync(nd.bar, nd.threads);  // slast is written again by the next tile
+    }
+    const uint32_t chs = __reduce_add_sync(kFull, counted ? fo + 1u : 0u);
+    if (lane == 0) ev += chs;
     if (bval) {
       if (R == col0) {
         a.pruned_num[b] = K;
@@ -428,8 +540,6 @@ __global__ void __launch_bounds__(kTile, S == 2 ? 4 : 3) k_prune_tc(const PruneA
       }
       if (my_kept != kNone) {
         a.pruned[b * a.p + my_kept] = x;
-        if (a.pruned_dist)  // a NaN when the list held no chain's distance (the node itself)
-          a.pruned_dist[b * a.p + my_kept] = valid ? dist : __uint_as_float(0x7FFFFFFFu);
         atomicAdd(a.indeg + x, 1u);
       }
     }
@@ -457,7 +567,7 @@ __global__ void __launch_bounds__(kTile, S == 2 ? 4 : 3) k_prune_tc(const PruneA
 
 template <bool HALF, uint32_t S>
 cudaError_t launch_s(const PruneArgs& a, const TcShape& sh, int num_sms, cudaStream_t st) {
-  const size_t smem = smem_bytes(S, sh);
+  const size_t smem = smem_bytes(S);
   auto kern = k_prune_tc<HALF, S>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
@@ -489,28 +599,36 @@ cudaError_t launch_s(const PruneArgs& a, const TcShape& sh, int num_sms, cudaStr
   return cudaGetLastError();
 }
 
+cudaError_t launch_list_dists(const float* base, uint64_t n, uint32_t d, const uint32_t* lists,
+                              uint32_t c, uint32_t* keys, int num_sms, cudaStream_t st) {
+  uint64_t blocks = (n + 7) / 8;
+  const uint64_t cap = static_cast<uint64_t>(num_sms) * 8;
+  if (blocks > cap) blocks = cap;
+  auto kern = c == 64 ? k_list_dists<2> : c == 96 ? k_list_dists<3> : k_list_dists<4>;
+  if (c != 64 && c != 96 && c != 128) return cudaErrorInvalidValue;
+  kern<<<static_cast<unsigned>(blocks), 256, 0, st>>>(base, n, d, lists, keys);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_prune_screen(const PruneArgs& a, int num_sms, size_t smem_optin,
                                 cudaStream_t st) {
-  if (!screen_supported(a.c, a.d, a.strict) || !a.norms ||
-      (reinterpret_cast<uintptr_t>(a.base) % 16) != 0)
+  if (!screen_supported(a.c, a.d, a.strict) || !a.norms || !a.rows16 || !a.cand_dist ||
+      (reinterpret_cast<uintptr_t>(a.base) % 16) != 0 ||
+      (reinterpret_cast<uintptr_t>(a.rows16) % 16) != 0)
     return cudaErrorInvalidValue;
   if (a.n == 0) return cudaSuccess;
   if (a.n > 0x7FFFFFFFull) return cudaErrorInvalidValue;
   TcShape sh{};
   sh.cap = a.c <= 64 ? 64u : 128u;
-  sh.nk = (a.d + kCk - 1) / kCk;
-  sh.dpad = sh.nk * kCk;
+  sh.dp = screen_row(a.d);
+  sh.nk = (sh.dp + kCk - 1) / kCk;
   const uint32_t per_tile = kTile / sh.cap;
   sh.tiles = (a.n + per_tile - 1) / per_tile;
   uint32_t s = a.stages ? a.stages : kDefaultStages;
   if (s < kMinStages) s = kMinStages;
   if (s > kMaxStages) s = kMaxStages;
-  auto fit = [&](uint32_t k) {
-    sh.nbuf = (k - 1 + sh.nk - 1) / sh.nk + 1;  // tiles the copies run ahead, plus the current
-    return smem_bytes(k, sh) <= smem_optin;
-  };
-  while (s > kMinStages && !fit(s)) s--;
-  if (!fit(s)) return cudaErrorInvalidValue;
+  while (s > kMinStages && smem_bytes(s) > smem_optin) s--;
+  if (smem_bytes(s) > smem_optin) return cudaErrorInvalidValue;
   const bool half = a.screen_half != 0;
   switch (s) {
     case 2: return half ? launch_s<true, 2>(a, sh, num_sms, st) : launch_s<false, 2>(a, sh, num_sms, st);

@@ -39,12 +39,15 @@ bool screen_supported(uint32_t c, uint32_t d, int strict) {
 }
 
 // Per point: upper bounds of |x| and of |x - x^| + |x^_sub| (x^ = the 16-bit copy the screened
-// prune packs, x^_sub its subnormal part), read by k_prune_tc in place of per-candidate sums.
+// prune multiplies, x^_sub its subnormal part).
 // One warp per point.  The 1.0001 factor covers the FP32 sums' rounding for D <= 1024 and the
 // 1e-21 term their underflow (at most D * 2^-150 absolute, whose square root is below 1e-21).
+// Also writes the copies themselves, rows of screen_row(d) elements, the padding zero.
 template <bool HALF>
 __global__ void __launch_bounds__(256) k_screen_norms(const float* __restrict__ base, uint64_t n,
-                                                      uint32_t d, float2* __restrict__ out) {
+                                                      uint32_t d, uint32_t dp,
+                                                      float2* __restrict__ out,
+                                                      uint2* __restrict__ rows16) {
   const float min_normal = HALF ? 6.103515625e-05f : 1.17549435e-38f;  // 2^-14, 2^-126
   const uint32_t lane = lane_id();
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -52,19 +55,21 @@ __global__ void __launch_bounds__(256) k_screen_norms(const float* __restrict__ 
        i < n; i += nw) {
     const float4* r = reinterpret_cast<const float4*>(base + i * d);
     float nn = 0.f, ee = 0.f, ss = 0.f;
-    for (uint32_t k = lane; k < (d >> 2); k += 32) {
-      const float4 v = __ldg(r + k);
+    for (uint32_t k = lane; k < (dp >> 2); k += 32) {
+      const float4 v = k < (d >> 2) ? __ldg(r + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      uint32_t h[2];
       const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
       for (int t = 0; t < 4; t += 2) {
         float e0, e1;
-        pack2<HALF>(x[t], x[t + 1], e0, e1);
+        h[t / 2] = pack2<HALF>(x[t], x[t + 1], e0, e1);
         const float r0 = x[t] - e0, r1 = x[t + 1] - e1;  // the rounded values
         nn = fmaf(x[t], x[t], fmaf(x[t + 1], x[t + 1], nn));
         ee = fmaf(e0, e0, fmaf(e1, e1, ee));
         if (fabsf(r0) < min_normal) ss = fmaf(r0, r0, ss);
         if (fabsf(r1) < min_normal) ss = fmaf(r1, r1, ss);
       }
+      rows16[i * (dp >> 2) + k] = make_uint2(h[0], h[1]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -79,16 +84,18 @@ __global__ void __launch_bounds__(256) k_screen_norms(const float* __restrict__ 
 }
 
 cudaError_t launch_screen_norms(const float* base, uint64_t n, uint32_t d, uint32_t half,
-                                float2* out, int num_sms, cudaStream_t st) {
+                                float2* out, void* rows16, int num_sms, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  if (d == 0 || (d % 4) != 0 || !out) return cudaErrorInvalidValue;
+  if (d == 0 || (d % 4) != 0 || !out || !rows16) return cudaErrorInvalidValue;
+  const uint32_t dp = screen_row(d);
+  uint2* rows = static_cast<uint2*>(rows16);
   uint64_t blocks = (n + 7) / 8;
   const uint64_t cap = static_cast<uint64_t>(num_sms) * 8;
   if (blocks > cap) blocks = cap;
   if (half)
-    k_screen_norms<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(base, n, d, out);
+    k_screen_norms<true><<<static_cast<unsigned>(blocks), 256, 0, st>>>(base, n, d, dp, out, rows);
   else
-    k_screen_norms<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(base, n, d, out);
+    k_screen_norms<false><<<static_cast<unsigned>(blocks), 256, 0, st>>>(base, n, d, dp, out, rows);
   return cudaGetLastError();
 }
 

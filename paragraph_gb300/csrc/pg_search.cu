@@ -444,6 +444,16 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
       if (tpos < a.out_width) orow[tpos] = top_id[s] & kMaskedTomb;
     }
     if (cpos < a.out_width) orow[cpos] = cand_id & kMaskedTomb;
+    if (a.out_key) {  // for launch_list_dists: only stores here, since more code in this place made
+                      // the search loop's registers spill (300k x 512: 27.7 -> 32.5 ms)
+      uint32_t* krow = a.out_key + static_cast<uint64_t>(qid) * a.out_width;
+#pragma unroll
+      for (int s = 0; s < KM_S; s++) {
+        const uint32_t tpos = static_cast<uint32_t>(s) * 32u + lane + shift[s];
+        if (tpos < a.out_width) krow[tpos] = top_key[s];
+      }
+      if (cpos < a.out_width) krow[cpos] = newc ? cand_key : kNoKey;
+    }
   }
   if (lane == 0) {
     if (ev) atomicAdd(a.evals, ev);

@@ -617,6 +617,13 @@ __device__ __forceinline__ void smallest(const Key* __restrict__ seg, uint32_t d
       const uint32_t i = c0 + static_cast<uint32_t>(s) * 32u + lane;
       chunk[s] = (i < deg) ? seg[i] : ~Key(0);
     }
+    if (c0) {  // nothing below the last of the smallest so far (sources arrive mostly ascending)
+      const Key last = __shfl_sync(kFull, best[E - 1], 31);
+      bool below = false;
+#pragma unroll
+      for (int s = 0; s < E; s++) below |= chunk[s] < last;
+      if (!__any_sync(kFull, below)) continue;
+    }
     warp_sort_keys<E>(chunk);
     if (c0 == 0) {
 #pragma unroll
@@ -637,7 +644,8 @@ __device__ __forceinline__ void smallest(const Key* __restrict__ seg, uint32_t d
 // Reverse list of node p: the R smallest sources of its segment in ascending order, which is
 // what add_reverse (Gbuilder.cuh:1020-1038) stores when sources run in ascending order; the
 // count is min(in-degree, R).  The sort is sized to the segment (most hold a few entries);
-// segments longer than 128 keep a running 128-smallest set.
+// segments longer than 128 keep a running 128-smallest set and pass over chunks that cannot change
+// it (a hub of 1M x 200 has about 10^5 sources).
 template <bool DIST>
 __global__ void __launch_bounds__(256) k_reverse_lists(const uint32_t* __restrict__ offs,
                                                        const uint32_t* __restrict__ edges,

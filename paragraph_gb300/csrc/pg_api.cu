@@ -491,8 +491,8 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       sa.seed_dist = seed_dist;
       PG_CUDA(pg::launch_search(sa, sms, h->smem_optin, s));
       if (stage_events) PG_CUDA(cudaEventRecord(h->ev[2 + 3 * r], s));
-      PG_CUDA(cudaMemsetAsync(indeg, 0, n * 4, s));
-      pg::PruneArgs pr{};
+      pg::PruneArgs pr{};  // indeg: left zero by the reverse lists before
+
       pr.base = rows;
       pr.n = n;
       pr.d = d;

@@ -489,6 +489,7 @@ __global__ void __launch_bounds__(256) k_edge_dists(const float* __restrict__ ba
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr uint64_t kScanSmall = 4096;  // counts that one block scans
 // callers size the tile-sum buffers by kScanTileElems (pg_kernels.h)
 static_assert(kScanTile == kScanTileElems, "scan tile size must match kScanTileElems");
 
@@ -548,10 +549,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(uint32_t* __res
   if (threadIdx.x == 0) *total_out = carry;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in,
-                                                             uint64_t n,
+// Also leaves the counts and the cursors zero, for the next round and the scatter that follows.
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(uint32_t* __restrict__ in, uint64_t n,
                                                              const uint32_t* __restrict__ tile_off,
-                                                             uint32_t* __restrict__ out) {
+                                                             uint32_t* __restrict__ out,
+                                                             uint32_t* __restrict__ cursor) {
   __shared__ uint32_t ws[32];
   const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kScanTile + threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
@@ -564,9 +566,34 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
   uint32_t run = tile_off[blockIdx.x] + block_exclusive_scan(s, ws, nullptr);
 #pragma unroll
   for (int i = 0; i < kScanItems; i++) {
-    if (base + i < n) out[base + i] = run;
+    if (base + i < n) {
+      out[base + i] = run;
+      in[base + i] = 0;
+      cursor[base + i] = 0;
+    }
     run += v[i];
   }
+}
+
+// The same in one launch, one block, for small n (three launches cost more than the scan).
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(uint32_t* __restrict__ in, uint32_t n,
+                                                             uint32_t* __restrict__ out,
+                                                             uint32_t* __restrict__ cursor) {
+  __shared__ uint32_t ws[32];
+  uint32_t carry = 0;
+  for (uint32_t t0 = 0; t0 < n; t0 += kScanThreads) {
+    const uint32_t i = t0 + threadIdx.x;
+    const uint32_t v = i < n ? in[i] : 0u;
+    uint32_t total;
+    const uint32_t ex = block_exclusive_scan(v, ws, &total);
+    if (i < n) {
+      out[i] = carry + ex;
+      in[i] = 0;
+      cursor[i] = 0;
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) out[n] = carry;
 }
 
 // Every kept edge b -> p becomes the entry b in p's CSR segment (order fixed later by sorting);
@@ -928,17 +955,19 @@ cudaError_t launch_prune_reverse(const PruneArgs& a, bool phase1, int num_sms, c
 }
 
 cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_num, uint32_t p_len,
-                               uint64_t n, const uint32_t* indeg, uint32_t* offs,
+                               uint64_t n, uint32_t* indeg, uint32_t* offs,
                                uint32_t* tile_sums, uint32_t* cursor, uint32_t* edges,
                                int num_sms, cudaStream_t st, uint64_t rows,
                                const uint32_t* order, const float* pruned_dist) {
   if (rows == 0) rows = n;
-  const uint32_t tiles = static_cast<uint32_t>((n + kScanTile - 1) / kScanTile);
-  k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(indeg, n, tile_sums);
-  k_scan_tile_sums<<<1, kScanThreads, 0, st>>>(tile_sums, tiles, offs + n);
-  k_scan_apply<<<tiles, kScanThreads, 0, st>>>(indeg, n, tile_sums, offs);
-  cudaError_t e = cudaMemsetAsync(cursor, 0, n * sizeof(uint32_t), st);
-  if (e != cudaSuccess) return e;
+  if (n <= kScanSmall) {
+    k_scan_small<<<1, kScanThreads, 0, st>>>(indeg, static_cast<uint32_t>(n), offs, cursor);
+  } else {
+    const uint32_t tiles = static_cast<uint32_t>((n + kScanTile - 1) / kScanTile);
+    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(indeg, n, tile_sums);
+    k_scan_tile_sums<<<1, kScanThreads, 0, st>>>(tile_sums, tiles, offs + n);
+    k_scan_apply<<<tiles, kScanThreads, 0, st>>>(indeg, n, tile_sums, offs, cursor);
+  }
   auto scatter = pruned_dist ? k_scatter_reverse<true> : k_scatter_reverse<false>;
   scatter<<<grid_for(rows, 256, num_sms, 8), 256, 0, st>>>(pruned, pruned_num, pruned_dist, p_len,
                                                            rows, offs, cursor, edges, order);

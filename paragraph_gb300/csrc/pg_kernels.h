@@ -207,12 +207,12 @@ cudaError_t launch_prune_reverse(const PruneArgs& a, bool phase1, int num_sms, c
 // Reverse edges as CSR over n destinations: offs = exclusive scan of indeg, edges grouped by
 // destination holding the source row index.  `rows` pruned rows are scanned (0 = n).
 cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_num, uint32_t p_len,
-                               uint64_t n, const uint32_t* indeg, uint32_t* offs,
+                               uint64_t n, uint32_t* indeg, uint32_t* offs,
                                uint32_t* tile_sums, uint32_t* cursor, uint32_t* edges,
                                int num_sms, cudaStream_t st, uint64_t rows = 0,
                                const uint32_t* order = nullptr,
                                const float* pruned_dist = nullptr);
-// With pruned_dist / rev_dist every edge carries its distance (edges: 8 bytes each).
+// indeg is left zero.  With pruned_dist / rev_dist every edge carries its distance (edges: 8 bytes each).
 // With order / place (relocated builds) the edges hold original ids, which decide which sources a
 // list keeps and their sequence, and the lists hold places.
 cudaError_t launch_reverse_lists(const uint32_t* offs, const uint32_t* edges, uint64_t n,

@@ -72,3 +72,26 @@ def test_prune_and_merge_equal_oracle(pg, d, c, p, r, strict):
     assert ev == ref.evals
     assert np.array_equal(_u32(out), want)
     assert mev == want_ev
+
+
+@pytest.mark.parametrize("n", [1, 31, 1025, 4096, 4097, 8193])  # one-block scans and tiled ones
+@pytest.mark.parametrize("r", [7, 111])
+def test_reverse_lists_of_hubs_equal_oracle(pg, n, r):
+    rng = np.random.default_rng(n)
+    base = rng.standard_normal((n, 8)).astype(np.float32)
+    base[0] *= 50.0  # a hub: nearest for about half of the nodes
+    graph = rng.integers(0, n, (n, 6)).astype(np.uint32)
+    graph[:, 2] = 0
+    graph[rng.permutation(n), 3] = rng.integers(0, max(1, n // 50), n)
+    ref = oracle.prune_reverse(base, graph, 6, r, False)
+    pruned = torch.full((n, 6), -1, dtype=torch.int32, device="cuda")
+    rev = torch.full((n, r), -1, dtype=torch.int32, device="cuda")
+    pnum, rnum = torch.empty((2, n), dtype=torch.int32, device="cuda")
+    with pg.Handle(0) as h:
+        for _ in range(2):  # the second call finds the workspace that the first one left
+            h.prune_reverse(_dev(base), _dev(graph), pruned, pnum, rev, rnum, False)
+    assert np.array_equal(_u32(pnum), ref.pruned_num)
+    assert np.array_equal(_u32(rnum), ref.reverse_num)
+    want = np.where(np.arange(r)[None, :] < ref.reverse_num[:, None], ref.reverse, 0)
+    got = np.where(np.arange(r)[None, :] < ref.reverse_num[:, None], _u32(rev), 0)
+    assert np.array_equal(got, want)

@@ -405,6 +405,9 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     }
     if (stage_events) PG_CUDA(cudaEventRecord(h->ev[15], s));
 
+    const uint32_t half = p->screen == PG_SCREEN_FP16;
+    if (screened) PG_CUDA(pg::launch_screen_norms(rows, n, d, half, norms, rows16, sms, s));
+
     // K0 projection winners; K1+K2 phase-1 prune (rows read from gt through the winner)
     PG_CUDA(pg::launch_match_winner(gt, q, p->gt_k, n, winner, h->d_status, sms, s, d_seg, d_qseg,
                                     seg_count, place));
@@ -431,6 +434,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     pa.qseg_off = d_qseg;
     pa.seg_count = seg_count;
     pa.place = place;
+    pa.norms = norms;
     PG_CUDA(pg::launch_prune_reverse(pa, true, sms, s));
     PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->proj_pruned, n, indeg, offs, tsum, cursor, edges,
                                    sms, s, 0, order, pdist));
@@ -509,13 +513,11 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
       pr.status = h->d_status;
       pr.rescored = cnt + C_RESCORED + r;
       pr.stages = h->tune.screen_stages;
-      pr.screen_half = p->screen == PG_SCREEN_FP16;
+      pr.screen_half = half;
       pr.norms = norms;
       pr.rows16 = rows16;
       pr.cand_dist = reinterpret_cast<const float*>(sdist);
       if (screened) {
-        if (r == 0)
-          PG_CUDA(pg::launch_screen_norms(rows, n, d, pr.screen_half, norms, rows16, sms, s));
         PG_CUDA(pg::launch_list_dists(rows, n, d, sres, L, sdist, sms, s));
         PG_CUDA(pg::launch_prune_screen(pr, sms, h->smem_optin, s));
         PG_CUDA(pg::launch_edge_dists(rows, n, d, pruned, pnum, p->degree, pdist, sms, s));

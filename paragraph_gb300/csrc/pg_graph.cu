@@ -325,11 +325,12 @@ __device__ __forceinline__ void test_screened(NodeLists<W>* sm, const float* __r
 // fusion_prune_reverse_kernel_v0 (Gbuilder.cuh:1093-1244), one block of W warps per node of up to
 // 32 W candidates, a thread per candidate.  PHASE1 reads the candidate row of node b straight from
 // the winner's ground truth (the K0 row) instead of a materialised graph, and looks for nodes that
-// have a winner `look` (at most 32) at a time.  Bound by the latency of the chains.  Against one
+// have a winner `look` (at most 32) at a time; in screened builds its tests are decided as the
+// merge's are.  Bound by the latency of the chains.  Against one
 // warp per node, several candidates per lane and a scan whose window bookkeeping was serial: the
 // whole projection of 1000 x 200 0.33 -> 0.12 ms and of 120k x 512 4.2 -> 2.2 ms, both link prunes
 // of 120k x 512 (c = 64) 11.9 -> 10.7 ms.
-template <int W, bool PHASE1, bool WIDE>
+template <int W, bool PHASE1, bool SCREEN, bool WIDE>
 __device__ __forceinline__ void prune_node(const PruneArgs& a, NodeLists<W>* sm, uint64_t b,
                                            uint32_t w, uint32_t* ev) {
   using T = Team<W>;
@@ -379,7 +380,10 @@ __device__ __forceinline__ void prune_node(const PruneArgs& a, NodeLists<W>* sm,
   uint32_t checks = 0;
   uint32_t k = team_scan<W>(sm, a.n, end, a.p,
                             [&](const uint8_t* tl, uint32_t tn, uint32_t r) {
-                              test_exact<W, WIDE>(sm, a.base, a.d, tl, tn, r);
+                              if constexpr (SCREEN)
+                                test_screened<W>(sm, a.base, a.d, a.norms, tl, tn, r);
+                              else
+                                test_exact<W, WIDE>(sm, a.base, a.d, tl, tn, r);
                             },
                             &checks);
   if (T::lead()) {
@@ -413,7 +417,7 @@ __device__ __forceinline__ void prune_node(const PruneArgs& a, NodeLists<W>* sm,
 
 constexpr int kPruneWarps = 24;  // warps per SM (80 registers)
 
-template <int W, bool PHASE1, bool WIDE>
+template <int W, bool PHASE1, bool SCREEN, bool WIDE>
 __global__ void __launch_bounds__(32 * W, kPruneWarps / W) k_prune_reverse(PruneArgs a, uint32_t look) {
   __shared__ NodeLists<W> sm;
   uint32_t part = 0;
@@ -429,14 +433,14 @@ __global__ void __launch_bounds__(32 * W, kPruneWarps / W) k_prune_reverse(Prune
       if (threadIdx.x < 32 && in && w == kTomb) a.pruned_num[b] = 0;  // nobody's top-1
       for (; todo; todo &= todo - 1u) {
         const int l = __ffs(static_cast<int>(todo)) - 1;
-        prune_node<W, true, WIDE>(a, &sm, b0 + l, __shfl_sync(kFull, w, l), &part);
+        prune_node<W, true, SCREEN, WIDE>(a, &sm, b0 + l, __shfl_sync(kFull, w, l), &part);
         ev += part;
         part = 0;
       }
     }
   } else {
     for (uint64_t b = blockIdx.x; b < a.n; b += gridDim.x) {
-      prune_node<W, false, WIDE>(a, &sm, b, kTomb, &part);
+      prune_node<W, false, SCREEN, WIDE>(a, &sm, b, kTomb, &part);
       ev += part;
       part = 0;
     }
@@ -940,7 +944,10 @@ static cudaError_t launch_prune_w(const PruneArgs& a, int num_sms, cudaStream_t 
   uint64_t look = P1 ? a.n / (static_cast<uint64_t>(num_sms) * per_sm) : 1;
   look = look < 1 ? 1 : look > 32 ? 32 : look;
   const unsigned grid = grid_for(a.n, static_cast<int>(look), num_sms, per_sm);
-  auto kern = wide_rows(a.base, a.d) ? k_prune_reverse<W, P1, true> : k_prune_reverse<W, P1, false>;
+  auto kern = wide_rows(a.base, a.d) ? k_prune_reverse<W, P1, false, true>
+                                     : k_prune_reverse<W, P1, false, false>;
+  if constexpr (P1)
+    if (a.norms) kern = k_prune_reverse<W, P1, true, true>;
   kern<<<grid, 32 * W, 0, st>>>(a, static_cast<uint32_t>(look));
   return cudaGetLastError();
 }

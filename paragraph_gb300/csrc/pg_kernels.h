@@ -35,7 +35,7 @@ struct PruneArgs {
   // depend on it
   uint32_t stages;
   uint32_t screen_half;  // screened kernel: FP16 operands instead of BF16
-  // screened kernel: per point (|x|, |x - x^| + |x^_sub|) upper bounds and the 16-bit rows from
+  // screened builds: per point (|x|, |x - x^| + |x^_sub|) upper bounds (phase 1 too) and the 16-bit rows from
   // launch_screen_norms with the same screen_half, and the candidates' distances (n x c) from
   // launch_list_dists
   const float2* norms;

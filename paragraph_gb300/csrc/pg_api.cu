@@ -1649,20 +1649,26 @@ int pg_ground_truth(pg_handle h, const float* d_base, uint64_t n, uint32_t d,
   if (k < 1 || k > pg::gt_max_k()) return fail(PG_EINVAL, "k=%u must be in [1, %u]", k, pg::gt_max_k());
   std::lock_guard<std::mutex> lk(h->mu);
   PG_CUDA(cudaSetDevice(h->device));
-  const pg::GtPlan plan = pg::gt_plan(n, nq, d, h->num_sms, h->smem_optin);
-  int rc = ensure_ws(h, pg::gt_workspace_bytes(plan, n, nq));
-  if (rc) return rc;
-  PG_CUDA(cudaMemsetAsync(h->d_status, 0, 4, h->stream));
-  // diagnostics in the counters' spare words: the first query's margin, max |x^|, max |x - x^|
-  float* diag = reinterpret_cast<float*>(h->d_counters + 60);
-  const int r = pg::ground_truth(plan, d_base, n, d, d_queries, nq, k, d_out, h->ws,
-                                 h->d_status, h->num_sms, h->stream, diag);
-  if (r < 0) return fail(PG_ECUDA, "ground truth: %s", cudaGetErrorString(static_cast<cudaError_t>(-r)));
-  if (r > 0) return fail(PG_ECUDA, "ground truth: cannot encode a TMA tensor map");
-  PG_CUDA(cudaMemcpyAsync(h->h_status, h->d_status, 4, cudaMemcpyDeviceToHost, h->stream));
-  PG_CUDA(cudaMemcpyAsync(h->h_counters + 60, diag, 12, cudaMemcpyDeviceToHost, h->stream));
-  PG_CUDA(cudaStreamSynchronize(h->stream));
-  const uint32_t st = *h->h_status;
+  uint32_t st = 0;
+  for (bool sampled : {true, false}) {
+    const pg::GtPlan plan = pg::gt_plan(n, nq, d, k, sampled, h->num_sms, h->smem_optin);
+    int rc = ensure_ws(h, pg::gt_workspace_bytes(plan, n, nq));
+    if (rc) return rc;
+    PG_CUDA(cudaMemsetAsync(h->d_status, 0, 4, h->stream));
+    // diagnostics in the counters' spare words: the first query's margin, max |x^|, max |x - x^|
+    float* diag = reinterpret_cast<float*>(h->d_counters + 60);
+    const int r = pg::ground_truth(plan, d_base, n, d, d_queries, nq, k, d_out, h->ws,
+                                   h->d_status, h->num_sms, h->stream, diag);
+    if (r < 0)
+      return fail(PG_ECUDA, "ground truth: %s", cudaGetErrorString(static_cast<cudaError_t>(-r)));
+    if (r > 0) return fail(PG_ECUDA, "ground truth: cannot encode a TMA tensor map");
+    PG_CUDA(cudaMemcpyAsync(h->h_status, h->d_status, 4, cudaMemcpyDeviceToHost, h->stream));
+    PG_CUDA(cudaMemcpyAsync(h->h_counters + 60, diag, 12, cudaMemcpyDeviceToHost, h->stream));
+    PG_CUDA(cudaStreamSynchronize(h->stream));
+    st = *h->h_status;
+    // a sampled threshold let too many candidates through: once more with every tile
+    if (plan.step == 1 || st != (1u << 6)) break;
+  }
   const float* dg = reinterpret_cast<const float*>(h->h_counters + 60);
   if (st & (1u << 4)) return fail(PG_EUNSUPPORTED, "ground truth: a value beyond the FP16 range");
   if (st & (1u << 6))

@@ -14,16 +14,19 @@
 //      + g (|q^| max|x^|), with g covering the FP32 accumulation (d' * 2^-22, four times the
 //      IEEE unit roundoff, for the tensor core's accumulation);
 //   4. pass 1 (k_gt_tc<kMax>): the maximum screened score of every group of base rows per query
-//      (disjoint groups, about 4096 or more of them); the k-th largest group maximum theta_q is
-//      the score of k distinct base rows, so theta_q <= t_k, the k-th largest screened score of
-//      the row (k_gt_theta);
+//      (disjoint groups, about 4096 or more of them), over a sample of the base tiles where it is
+//      large; the k-th largest group maximum theta_q is the score of k distinct base rows, so
+//      theta_q <= t_k, the k-th largest screened score of the row (k_gt_theta);
 //   5. pass 2 (k_gt_tc<kFilter>): every base row with s^ >= theta_q - 2 E_q is a candidate --
 //      a superset of {s^ >= t_k - 2 E_q}, which holds the true top k (a true top-k member has
 //      s^ >= s_k - E_q and s_k >= t_k - E_q);
 //   6. k_gt_final: the candidates with s^ >= t_k - 2 E_q, exact FP64 inner products, sorted by
 //      (score desc, id asc).
 // With groups many enough that the top k fall in nearly distinct groups, theta_q sits just
-// below t_k and a query keeps about 1.1 k candidates.
+// below t_k and a query keeps about 1.1 k candidates.  From a sample of every step-th tile it keeps
+// about 1.1 k step, which k_gt_narrow brings back to 1.1 k; pass 1 then costs 1 / step of pass 2.
+// Data on which a sampled threshold lets through more than the selection holds (near rows placed to
+// miss the sample) are done again with every tile.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -415,15 +418,102 @@ cudaError_t launch_final(const GtArgs& f, int num_sms, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima (-inf when
-// there are fewer than k groups: every base row is then a candidate).
-// A histogram of kThetaBins equal steps between the row's smallest and largest maximum finds the
-// step that holds the k-th largest; its few maxima are then gathered and ranked.  A step with more
-// than kThetaBins of them (an outlier far above the rest) is divided again.  The maxima spread over
-// the steps, so the shared-memory counters see few collisions and three passes over the row mostly
-// do: 3.4 -> 1.6 ms for 250k rows of 4700 maxima against a radix select, whose first of four
-// histograms collides on the sign and exponent.
+// The k-th largest of the values that `each` visits, given the smallest (mn) and largest (mx) of them
+// and at least k of them; one warp.  A histogram of kThetaBins equal steps between the two finds
+// the step that holds it; that step's few values are then gathered and ranked.  A step with more
+// than kThetaBins of them (an outlier far above the rest) is divided again.  The values spread over
+// the steps, so the shared-memory counters see few collisions, and three passes over them mostly
+// do.
 constexpr uint32_t kThetaBins = 512;
+template <class Each>
+__device__ float kth_largest(Each each, float mn, float mx, uint32_t k, uint32_t* hist,
+                             uint32_t* fill) {
+  const uint32_t lane = lane_id();
+  uint32_t need = k;  // its rank among the values in [mn, mx]
+  for (;;) {
+    const float scale = static_cast<float>(kThetaBins - 1) / (mx - mn);
+    // equal, or not divisible (a value out of range, which raised its error): all count
+    if (!(mx > mn) || !(scale > 0.0f && scale < INFINITY)) break;
+    const float low = mn, high = mx;
+    auto bin = [&](float v) {  // non-decreasing in v
+      return min(static_cast<uint32_t>((v - low) * scale), kThetaBins - 1);
+    };
+    for (uint32_t b = lane; b < kThetaBins; b += 32) hist[b] = 0;
+    __syncwarp();
+    each([&](float v) {
+      if (v >= low && v <= high) atomicAdd(hist + bin(v), 1u);
+    });
+    __syncwarp();
+    // lane l sums bins from the top: kThetaBins - 1 - 16 l downwards
+    constexpr uint32_t kPer = kThetaBins / 32;
+    uint32_t sum = 0;
+    for (uint32_t t = 0; t < kPer; t++) sum += hist[kThetaBins - 1 - (lane * kPer + t)];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= static_cast<uint32_t>(o)) incl += y;
+    }
+    const uint32_t excl = incl - sum;
+    const unsigned owner = __ballot_sync(kFull, excl < need && need <= incl);
+    const int src = __ffs(static_cast<int>(owner)) - 1;
+    uint32_t at = 0, above = 0, held = 0;
+    if (static_cast<int>(lane) == src) {
+      above = excl;
+      for (uint32_t t = 0; t < kPer; t++) {
+        at = kThetaBins - 1 - (lane * kPer + t);
+        held = hist[at];
+        if (above + held >= need) break;
+        above += held;
+      }
+    }
+    at = __shfl_sync(kFull, at, src);
+    above = __shfl_sync(kFull, above, src);
+    held = __shfl_sync(kFull, held, src);
+    need -= above;
+    __syncwarp();
+    if (held <= kThetaBins) {  // its values in the counters' place; the need-th largest of them
+      float* vals = reinterpret_cast<float*>(hist);
+      if (lane == 0) *fill = 0;
+      __syncwarp();
+      each([&](float v) {
+        if (v >= low && v <= high && bin(v) == at) vals[atomicAdd(fill, 1u)] = v;
+      });
+      __syncwarp();
+      mn = INFINITY;
+      for (uint32_t i = lane; i < held; i += 32) {
+        const float v = vals[i];
+        uint32_t gt = 0, eq = 0;
+        for (uint32_t j = 0; j < held; j++) {
+          gt += vals[j] > v ? 1u : 0u;
+          eq += vals[j] == v ? 1u : 0u;
+        }
+        if (gt < need && need <= gt + eq) mn = v;
+      }
+      for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+      __syncwarp();
+      break;
+    }
+    mn = INFINITY;
+    mx = -INFINITY;
+    each([&](float v) {
+      if (v >= low && v <= high && bin(v) == at) {
+        mn = fminf(mn, v);
+        mx = fmaxf(mx, v);
+      }
+    });
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+    }
+  }
+  return mn;
+}
+
+// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima (-inf when
+// there are fewer than k groups: every base row is then a candidate).  3.4 -> 1.6 ms for 250k rows of
+// 4700 maxima against a radix select, whose first of four histograms collides on the sign and
+// exponent.
 template <bool PAIRS>  // an even number of groups: rows start on 8 bytes
 __global__ void __launch_bounds__(256) k_gt_theta(const float* __restrict__ maxima,
                                                   uint32_t rows, uint32_t groups, uint32_t k,
@@ -470,85 +560,60 @@ __global__ void __launch_bounds__(256) k_gt_theta(const float* __restrict__ maxi
       if (lane == 0) lo[row] = -INFINITY;
       continue;
     }
-    uint32_t need = k;  // theta's rank among the maxima in [mn, mx]
-    for (;;) {
-      const float scale = static_cast<float>(kThetaBins - 1) / (mx - mn);
-      // equal, or not divisible (a value out of range, which raised its error): all count
-      if (!(mx > mn) || !(scale > 0.0f && scale < INFINITY)) break;
-      const float low = mn, high = mx;
-      auto bin = [&](float v) {  // non-decreasing in v
-        return min(static_cast<uint32_t>((v - low) * scale), kThetaBins - 1);
-      };
-      for (uint32_t b = lane; b < kThetaBins; b += 32) hist[b] = 0;
-      __syncwarp();
-      each([&](float v) {
-        if (v >= low && v <= high) atomicAdd(hist + bin(v), 1u);
-      });
-      __syncwarp();
-      // lane l sums bins from the top: kThetaBins - 1 - 16 l downwards
-      constexpr uint32_t kPer = kThetaBins / 32;
-      uint32_t sum = 0;
-      for (uint32_t t = 0; t < kPer; t++) sum += hist[kThetaBins - 1 - (lane * kPer + t)];
-      uint32_t incl = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, incl, o);
-        if (lane >= static_cast<uint32_t>(o)) incl += y;
-      }
-      const uint32_t excl = incl - sum;
-      const unsigned owner = __ballot_sync(kFull, excl < need && need <= incl);
-      const int src = __ffs(static_cast<int>(owner)) - 1;
-      uint32_t at = 0, above = 0, held = 0;
-      if (static_cast<int>(lane) == src) {
-        above = excl;
-        for (uint32_t t = 0; t < kPer; t++) {
-          at = kThetaBins - 1 - (lane * kPer + t);
-          held = hist[at];
-          if (above + held >= need) break;
-          above += held;
-        }
-      }
-      at = __shfl_sync(kFull, at, src);
-      above = __shfl_sync(kFull, above, src);
-      held = __shfl_sync(kFull, held, src);
-      need -= above;
-      __syncwarp();
-      if (held <= kThetaBins) {  // its values in the counters' place; the need-th largest of them
-        float* vals = reinterpret_cast<float*>(hist);
-        if (lane == 0) *fill = 0;
-        __syncwarp();
-        each([&](float v) {
-          if (v >= low && v <= high && bin(v) == at) vals[atomicAdd(fill, 1u)] = v;
-        });
-        __syncwarp();
-        mn = INFINITY;
-        for (uint32_t i = lane; i < held; i += 32) {
-          const float v = vals[i];
-          uint32_t gt = 0, eq = 0;
-          for (uint32_t j = 0; j < held; j++) {
-            gt += vals[j] > v ? 1u : 0u;
-            eq += vals[j] == v ? 1u : 0u;
-          }
-          if (gt < need && need <= gt + eq) mn = v;
-        }
-        for (int o = 16; o > 0; o >>= 1) mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
-        __syncwarp();
-        break;
-      }
-      mn = INFINITY;
-      mx = -INFINITY;
-      each([&](float v) {
-        if (v >= low && v <= high && bin(v) == at) {
-          mn = fminf(mn, v);
-          mx = fmaxf(mx, v);
-        }
-      });
-      for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
-      }
+    const float theta = kth_largest(each, mn, mx, k, hist, fill);
+    if (lane == 0) lo[row] = theta - band[row];
+  }
+}
+
+// After a sampled threshold: one warp per query keeps, of its candidates, those within 2 E_q of the
+// k-th largest screened score (all of them when there are no more than k), in the list's first half
+// and then its second.
+__global__ void __launch_bounds__(128) k_gt_narrow(uint64_t* __restrict__ cand,
+                                                   uint32_t* __restrict__ cand_cnt, uint32_t rows,
+                                                   uint32_t k, const float* __restrict__ band) {
+  __shared__ uint64_t buf_all[4][kGtCap];
+  __shared__ uint32_t hist_all[4][kThetaBins];
+  __shared__ uint32_t fill_all[4];
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  uint64_t* buf = buf_all[warp];
+  const uint64_t nw = static_cast<uint64_t>(gridDim.x) * 4;
+  for (uint64_t row = blockIdx.x * 4ull + warp; row < rows; row += nw) {
+    const uint32_t c0 = min(cand_cnt[2 * row], kGtCap / 2);
+    const uint32_t c1 = min(cand_cnt[2 * row + 1], kGtCap / 2);
+    const uint32_t cnt = c0 + c1;
+    if (cnt <= k) continue;
+    uint64_t* list = cand + row * kGtCap;
+    float mn = INFINITY, mx = -INFINITY;
+    for (uint32_t i = lane; i < cnt; i += 32) {
+      const uint64_t key = list[i < c0 ? i : kGtCap / 2 + (i - c0)];
+      buf[i] = key;
+      const float v = key_value(key);
+      mn = fminf(mn, v);
+      mx = fmaxf(mx, v);
     }
-    if (lane == 0) lo[row] = mn - band[row];
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+    }
+    __syncwarp();
+    auto each = [&](auto&& use) {
+      for (uint32_t i = lane; i < cnt; i += 32) use(key_value(buf[i]));
+    };
+    const float low = kth_largest(each, mn, mx, k, hist_all[warp], fill_all + warp) - band[row];
+    uint32_t kept = 0;
+    for (uint32_t i0 = 0; i0 < cnt; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      const uint64_t key = i < cnt ? buf[i] : 0;
+      const bool keep = i < cnt && key_value(key) >= low;
+      const unsigned m = __ballot_sync(kFull, keep);
+      if (keep) list[kept + __popc(m & ((1u << lane) - 1u))] = key;
+      kept += __popc(m);
+    }
+    if (lane == 0) {
+      cand_cnt[2 * row] = min(kept, kGtCap / 2);
+      cand_cnt[2 * row + 1] = kept - min(kept, kGtCap / 2);
+    }
+    __syncwarp();
   }
 }
 
@@ -601,6 +666,7 @@ struct Args {
   // group is `span` consecutive 32-column chunks of one thread (one half of each tile); span
   // == 0: a group is gs consecutive columns (gs < 32, for small n).
   uint32_t span, gs, groups;
+  uint32_t step;    // kMax: every step-th base tile is swept (1 in the other modes)
   float* maxima;    // kMax: nq x groups
   const float* lo;  // kFilter: nq thresholds
   uint64_t* cand;   // kFilter: nq x kGtCap keys, two halves of kGtCap / 2
@@ -663,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   constexpr uint32_t rows_per_tile = kRows * MT;
   const uint32_t q_tiles = (a.nq + rows_per_tile - 1) / rows_per_tile;
-  const uint32_t n_tiles = (a.n + BN - 1) / BN;
+  const uint32_t n_tiles = ((a.n + BN - 1) / BN + a.step - 1) / a.step;  // tiles swept
   constexpr uint32_t ncols = 2 * BN * MT;  // two accumulator buffers per M tile (512)
 
   if (threadIdx.x == 0) {
@@ -719,7 +785,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             bar_expect_tx(full + s, kStageBytes);
 #pragma unroll
             for (uint32_t r = 0; r < BN / kRows; r++)
-              tma_load(sB + s * kStageBytes + r * kBox, &tb, c * kChunk, bt * BN + r * kRows,
+              tma_load(sB + s * kStageBytes + r * kBox, &tb, c * kChunk, bt * a.step * BN + r * kRows,
                        full + s);
           }
       }
@@ -820,7 +886,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (uint32_t i = 0; i < 4; i++) {
           const uint32_t m = i / kCpt, ch = i % kCpt;
           if (!valid[m]) continue;
-          const uint32_t col0 = bt * BN + half * kHalf + ch * 32;
+          const uint32_t col0 = bt * a.step * BN + half * kHalf + ch * 32;
           const uint32_t inr = in_range(col0, a.n);
           if (MODE == kMax) {
             if (a.span) {
@@ -972,7 +1038,8 @@ uint32_t gt_max_k() { return 256; }
 
 uint32_t gt_max_dim() { return tc::kChunk * tc::kMaxKc; }
 
-GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, int num_sms, size_t smem_optin) {
+GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, uint32_t k, bool sampled, int num_sms,
+               size_t smem_optin) {
   GtPlan p{};
   p.dp = padded_dim(d);
   p.kc = k_boxes(p.dp);
@@ -983,11 +1050,18 @@ GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, int num_sms, size_t smem_opt
   // for small n groups of gs < 32 columns
   const uint64_t n_tiles = (n + p.bn - 1) / p.bn;
   const uint64_t chunks = n_tiles * (p.bn / 64);  // per thread
+  // A sample of the base, every step-th tile, gives a threshold too: the k-th largest of its group
+  // maxima is the score of k distinct rows.  Then about k step rows pass the filter, so step keeps
+  // them well inside the selection's room, and the sample keeps 16 k groups.
+  p.step = 1;
+  if (sampled && 2 * chunks >= 4096)
+    while (p.step < 8 && 2ull * p.step * k <= 560 && chunks / p.step >= 16ull * k) p.step *= 2;
+  const uint64_t swept = (n_tiles + p.step - 1) / p.step * (p.bn / 64);
   if (2 * chunks >= 4096) {
     p.span = 1;
-    while (2 * ((chunks + 2 * p.span - 1) / (2 * p.span)) >= 4096) p.span *= 2;
+    while (2 * ((swept + 2 * p.span - 1) / (2 * p.span)) >= 4096) p.span *= 2;
     p.gs = 0;
-    p.groups = static_cast<uint32_t>(2 * ((chunks + p.span - 1) / p.span));
+    p.groups = static_cast<uint32_t>(2 * ((swept + p.span - 1) / p.span));
   } else {
     p.span = 0;
     p.gs = 1;
@@ -1062,6 +1136,7 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
     a.span = plan.span;
     a.gs = plan.gs;
     a.groups = plan.groups;
+    a.step = plan.step;
     a.maxima = maxima;
     a.lo = lo;
     a.cand = cand;
@@ -1071,8 +1146,11 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
       return -static_cast<int>(e);
     auto theta = plan.groups % 2 ? k_gt_theta<false> : k_gt_theta<true>;
     theta<<<blocks_for(rows, 8, num_sms, 8), 256, 0, st>>>(maxima, rows, plan.groups, k, band, lo);
+    a.step = 1;
     if ((e = tc::launch<tc::kFilter>(ta, tb, a, num_sms, st)) != cudaSuccess)
       return -static_cast<int>(e);
+    if (plan.step > 1)
+      k_gt_narrow<<<blocks_for(rows, 4, num_sms, 12), 128, 0, st>>>(cand, cand_cnt, rows, k, band);
     GtArgs f{};
     f.base = base;
     f.queries = queries + q0 * d;
@@ -1138,6 +1216,7 @@ int screen_scores(const float* a, uint64_t na, const float* b, uint64_t nb, uint
   x.stages = tc::stages_for<tc::kBN>(x.kc, smem_optin);
   x.span = 1;
   x.groups = 1;
+  x.step = 1;
   x.dump = out;
   x.status = status;
   e = tc::launch<tc::kDump>(ta, tb, x, num_sms, st);

@@ -160,7 +160,8 @@ cudaError_t launch_fusion_final(const FusionArgs& a, int num_sms, cudaStream_t s
 // M tiles per CTA, the group size of the threshold pass and the queries per chunk.  The entry
 // points return 0, a negative cudaError_t, or 1 when a TMA tensor map cannot be encoded;
 // device-side problems set bits in *status (1 << 4: a value beyond the FP16 range, 1 << 6: a
-// query with more candidates than the selection holds, kErrWait: a bounded wait gave up).
+// query with more candidates than the selection holds -- with step > 1 the caller runs again
+// with a plan that samples nothing --, kErrWait: a bounded wait gave up).
 struct GtPlan {
   uint32_t dp;      // d rounded up to a multiple of 16 (FP16 rows zero-padded)
   uint32_t kc;      // 64-element K boxes per row: ceil(dp / 64)
@@ -169,11 +170,13 @@ struct GtPlan {
   uint32_t span;    // threshold pass: chunks of 32 columns per group (0: groups of gs columns)
   uint32_t gs;      // threshold pass, small n: columns per group
   uint32_t groups;  // groups per query
+  uint32_t step;    // threshold pass: every step-th base tile
   uint64_t cq;      // queries per chunk
 };
 uint32_t gt_max_k();
 uint32_t gt_max_dim();
-GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, int num_sms, size_t smem_optin);
+GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, uint32_t k, bool sampled, int num_sms,
+               size_t smem_optin);
 size_t gt_workspace_bytes(const GtPlan& p, uint64_t n, uint64_t nq);
 int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
                  const float* queries, uint64_t nq, uint32_t k, uint32_t* out, char* ws,

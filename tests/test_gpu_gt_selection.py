@@ -1,5 +1,6 @@
 """Ground-truth selection where its parts can go wrong: long candidate lists, runs of equal and of
-nearly equal scores, one maximum far above the rest, odd group counts, rows off a 16-byte boundary.
+nearly equal scores, one maximum far above the rest, odd group counts, rows off a 16-byte boundary,
+a sample of the base that misses the nearest rows.
 Ids equal the FP64 oracle's."""
 import numpy as np
 import pytest
@@ -26,14 +27,17 @@ def _base(kind, n, d, rng):
     elif kind == "close":  # neighbours differ in the last bits of one coordinate
         base[1::2] = base[0:n - n % 2:2]
         base[1::2, 0] = np.nextafter(base[1::2, 0], np.float32(9))
+    elif kind == "missed":  # the sampled tiles of a large base hold none of the nearest rows
+        base[(np.arange(n) // 256) % 8 != 0] *= 2.0
     elif kind == "outlier":  # the other maxima fall into one step of the first division
         base[n // 3] *= 20.0
     return np.ascontiguousarray(base)
 
 
-@pytest.mark.parametrize("kind", ["plain", "copies", "close", "outlier"])
+@pytest.mark.parametrize("kind", ["plain", "copies", "close", "outlier", "missed"])
 @pytest.mark.parametrize("n,nq,d,k", [(701, 33, 36, 256), (5003, 129, 200, 100),
-                                      (20_481, 9, 64, 128), (140_000, 3, 16, 10)])
+                                      (20_481, 9, 64, 128), (140_000, 3, 16, 10),
+                                      (270_000, 5, 8, 128)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_selection_equals_oracle(pg, kind, n, nq, d, k, shift):
     if kind == "copies":

@@ -161,7 +161,8 @@ struct Node {
     first = kNone;
     for (uint32_t w = 0; w < nw; w++) {
       const uint32_t m = x[w];
-      if (m && first == kNone) first = 32u * w + static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
+      if (m && first == kNone)
+        first = 32u * w + static_cast<uint32_t>(__ffs(static_cast<int>(m)) - 1);
       c += __popc(m);
     }
     return c;
@@ -204,7 +205,8 @@ __device__ __forceinline__ void feed_issue(Feed& f, const PruneArgs& a, const Tc
       const uint32_t rr = (R & ~31u) + 4u * i + (lane >> 3);  // tile row copied by this lane
       const uint32_t xr = __shfl_sync(kFull, f.x, 4u * i + (lane >> 3));
       if (xr != kNone && j < pieces)
-        cp16(st + rr * 128u + ((j ^ (rr & 7u)) << 4), src + static_cast<uint64_t>(xr) * (2u * sh.dp));
+        cp16(st + rr * 128u + ((j ^ (rr & 7u)) << 4),
+             src + static_cast<uint64_t>(xr) * (2u * sh.dp));
     }
     if (++f.kc == sh.nk) {
       f.kc = 0;
@@ -215,30 +217,39 @@ __device__ __forceinline__ void feed_issue(Feed& f, const PruneArgs& a, const Tc
   cp_commit();
 }
 
-// FP32 inner products of row r with the rows x of the lanes that `want` one, each valid in its lane:
-// four at a time, eight lanes per row, so that the loads are whole 128-byte lines.
+__device__ __forceinline__ float4 ldg4(const float* p) {
+  return __ldg(reinterpret_cast<const float4*>(p));
+}
+__device__ __forceinline__ void fma4(float4& s, const float4 u, const float4 v) {
+  s.x = fmaf(u.x, v.x, s.x);
+  s.y = fmaf(u.y, v.y, s.y);
+  s.z = fmaf(u.z, v.z, s.z);
+  s.w = fmaf(u.w, v.w, s.w);
+}
+__device__ __forceinline__ float sum4(const float4 s) { return (s.x + s.y) + (s.z + s.w); }
+
+// FP32 inner products of row r with the rows x of the lanes that `want` one, each valid in its
+// lane.  Loads are whole 128-byte lines.  Four rows at a time, eight lanes each; with WHOLE the last
+// one or two take the whole warp, which holds a row of 512 floats in one round of loads.  That is
+// the usual case in the prune, whose scan waits for it: round 2 of 1M x 512 97.6 -> 87.0 ms, but of
+// 1M x 200 9.0 -> 9.5 (the larger kernel), hence only for rows over 256 floats.
+template <bool WHOLE>
 __device__ __forceinline__ float warp_dots(const float* __restrict__ base, uint32_t d, uint32_t r,
                                            uint32_t x, bool want) {
   const uint32_t lane = threadIdx.x & 31u, g = lane >> 3, m = lane & 7u;
   unsigned todo = __ballot_sync(kFull, want);
   const float* rrow = base + static_cast<uint64_t>(r) * d;
   float mine = 0.f;
-  while (todo) {
+  constexpr uint32_t few = WHOLE ? 2 : 0;
+  while (__popc(todo) > few) {
     unsigned t = todo;
     for (uint32_t i = 0; i < g; i++) t &= t - 1u;  // group g takes the g-th lane, or repeats one
     const int src = __ffs(static_cast<int>(t ? t : todo)) - 1;
     const float* xrow = base + static_cast<uint64_t>(__shfl_sync(kFull, x, src)) * d;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-    for (uint32_t c = 4u * m; c < d; c += 32) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(rrow + c));
-      const float4 v = __ldg(reinterpret_cast<const float4*>(xrow + c));
-      s.x = fmaf(u.x, v.x, s.x);
-      s.y = fmaf(u.y, v.y, s.y);
-      s.z = fmaf(u.z, v.z, s.z);
-      s.w = fmaf(u.w, v.w, s.w);
-    }
-    float v = (s.x + s.y) + (s.z + s.w);
+    for (uint32_t c = 4u * m; c < d; c += 32) fma4(s, ldg4(rrow + c), ldg4(xrow + c));
+    float v = sum4(s);
     v += __shfl_xor_sync(kFull, v, 4);
     v += __shfl_xor_sync(kFull, v, 2);
     v += __shfl_xor_sync(kFull, v, 1);
@@ -246,6 +257,28 @@ __device__ __forceinline__ float warp_dots(const float* __restrict__ base, uint3
     const float got = __shfl_sync(kFull, v, static_cast<int>((rank & 3u) << 3));
     if (((todo >> lane) & 1u) && rank < 4) mine = got;
     for (uint32_t i = 0; i < 4; i++) todo &= todo - 1u;  // 0 stays 0
+  }
+  if (WHOLE && todo) {
+    const int l0 = __ffs(static_cast<int>(todo)) - 1;
+    const int l1 = 31 - __clz(static_cast<int>(todo));
+    const float* x0 = base + static_cast<uint64_t>(__shfl_sync(kFull, x, l0)) * d;
+    const float* x1 = base + static_cast<uint64_t>(__shfl_sync(kFull, x, l1)) * d;
+    float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
+#pragma unroll 4
+    for (uint32_t c = 4u * lane; c < d; c += 128) {
+      const float4 u = ldg4(rrow + c);
+      fma4(s0, u, ldg4(x0 + c));
+      fma4(s1, u, ldg4(x1 + c));
+    }
+    // the lower half of the warp finishes the first, the upper half the second
+    const float a = sum4(s0), b = sum4(s1);
+    const bool up = lane >= 16;
+    float v = (up ? b : a) + __shfl_xor_sync(kFull, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    const float v0 = __shfl_sync(kFull, v, 0), v1 = __shfl_sync(kFull, v, 16);
+    if (static_cast<int>(lane) == l0) mine = v0;
+    if (static_cast<int>(lane) == l1) mine = l0 == l1 ? v0 : v1;
   }
   return mine;
 }
@@ -296,7 +329,7 @@ __global__ void __launch_bounds__(256) k_list_dists(const float* __restrict__ ba
         }
         if (key[e] == kNoKey) key[e] = ks[at];
         const bool want = key[e] == kNoKey;
-        const float s32 = warp_dots(base, d, static_cast<uint32_t>(b), id[e], want);
+        const float s32 = warp_dots<false>(base, d, static_cast<uint32_t>(b), id[e], want);
         if (want) key[e] = order_key(-s32);
       }
     }
@@ -306,7 +339,7 @@ __global__ void __launch_bounds__(256) k_list_dists(const float* __restrict__ ba
   }
 }
 
-template <bool HALF, uint32_t S>
+template <bool HALF, bool LONG, uint32_t S>
 __global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneArgs a,
                                                                    const TcShape sh) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -483,7 +516,7 @@ __global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneA
       }
       const uint32_t nun = __popc(__ballot_sync(kFull, !sure));
       if (nun) {  // inside the 16-bit margin: FP32 products, exact chains inside theirs (or NaN)
-        const float s32 = warp_dots(a.base, d, ri, x, !sure && valid && other);
+        const float s32 = warp_dots<LONG>(a.base, d, ri, x, !sure && valid && other);
         if (!sure) {
           if (valid && other) {
             const float dhat = -s32;
@@ -565,10 +598,10 @@ __global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneA
 
 }  // namespace
 
-template <bool HALF, uint32_t S>
+template <bool HALF, bool LONG, uint32_t S>
 cudaError_t launch_s(const PruneArgs& a, const TcShape& sh, int num_sms, cudaStream_t st) {
   const size_t smem = smem_bytes(S);
-  auto kern = k_prune_tc<HALF, S>;
+  auto kern = k_prune_tc<HALF, LONG, S>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
@@ -597,6 +630,16 @@ cudaError_t launch_s(const PruneArgs& a, const TcShape& sh, int num_sms, cudaStr
   if (blocks > sh.tiles) blocks = sh.tiles;
   kern<<<static_cast<unsigned>(blocks), kTile, smem, st>>>(a, sh);
   return cudaGetLastError();
+}
+
+template <uint32_t S>
+cudaError_t launch_half(const PruneArgs& a, const TcShape& sh, bool half, bool rows512, int num_sms,
+                        cudaStream_t st) {
+  if (rows512)
+    return half ? launch_s<true, true, S>(a, sh, num_sms, st)
+                : launch_s<false, true, S>(a, sh, num_sms, st);
+  return half ? launch_s<true, false, S>(a, sh, num_sms, st)
+              : launch_s<false, false, S>(a, sh, num_sms, st);
 }
 
 cudaError_t launch_list_dists(const float* base, uint64_t n, uint32_t d, const uint32_t* lists,
@@ -629,11 +672,11 @@ cudaError_t launch_prune_screen(const PruneArgs& a, int num_sms, size_t smem_opt
   if (s > kMaxStages) s = kMaxStages;
   while (s > kMinStages && smem_bytes(s) > smem_optin) s--;
   if (smem_bytes(s) > smem_optin) return cudaErrorInvalidValue;
-  const bool half = a.screen_half != 0;
+  const bool half = a.screen_half != 0, rows512 = a.d > 256;
   switch (s) {
-    case 2: return half ? launch_s<true, 2>(a, sh, num_sms, st) : launch_s<false, 2>(a, sh, num_sms, st);
-    case 3: return half ? launch_s<true, 3>(a, sh, num_sms, st) : launch_s<false, 3>(a, sh, num_sms, st);
-    default: return half ? launch_s<true, 4>(a, sh, num_sms, st) : launch_s<false, 4>(a, sh, num_sms, st);
+    case 2: return launch_half<2>(a, sh, half, rows512, num_sms, st);
+    case 3: return launch_half<3>(a, sh, half, rows512, num_sms, st);
+    default: return launch_half<4>(a, sh, half, rows512, num_sms, st);
   }
 }
 

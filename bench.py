@@ -211,9 +211,25 @@ def gpu_workload(args, device, queries: bool = False):
 # (profiles/search_dram_1Mx200_1Mx512cos.md): round 1 over the projection, round 2 over the link
 # graph.  Keys: (n, d, M, L, cosine).
 SEARCH_DRAM_BYTES = {
-    (1_000_000, 200, 32, 64, False): (1_217_476_352, 1_182_223_104),
-    (1_000_000, 512, 48, 96, True): (143_634_611_456, 870_972_185_088),
+    (1_000_000, 200, 32, 64, False): (1_507_496_960, 1_456_794_880),
+    (1_000_000, 512, 48, 96, True): (12_612_684_288, 23_788_843_520),
 }
+
+
+def build_launches(n, d, params, segments=0):
+    """Kernel launches of one build.  Once: the seed pre-pass, K0, the phase-1 prune; the copy of
+    the base in key order (three, and two to restore the results) when the base takes 32 MB to
+    32 GB, else for sub-indexes two to localize; when screened, the norm pre-pass.  Reverse CSR of
+    each prune: scan (one block up to 4096 points, else three), scatter, lists; then two merges
+    (short and long lists).  Per link round: search and prune, and when screened the distances of
+    the list entries and of the kept edges."""
+    rounds = params.link_rounds
+    screened = params.screen != 0 and params.km + params.kp * params.kd <= 128
+    reverse_and_merge = (1 if n <= 4096 else 3) + 2 + 2
+    relocated = rounds > 0 and 32 << 20 <= n * d * 4 <= 32 << 30 and segments <= 2048
+    count = 2 + reverse_and_merge + rounds * (2 + reverse_and_merge + (2 if screened else 0))
+    count += (1 if rounds else 0) + (1 if screened else 0)
+    return count + (5 if relocated else 2 if segments else 0)
 
 
 def search_roofline(st, args, peak_gbs, peak_kind, rounds):
@@ -221,9 +237,9 @@ def search_roofline(st, args, peak_gbs, peak_kind, rounds):
     evaluation after the 32 seeds gathers one 4*D-byte row plus its 4-byte id, every iteration
     reads Kp*Kd = 32 graph ids, and the launch reads each query row and its 32 seed distances once
     and writes n*L ids.  The seed distances are computed once per build by the seed pre-pass
-    (k_seed_dists, timed inside round 1's stage: it reads the n query rows and writes n*32
-    distances), so no search launch gathers a seed row.  The reported launch is the last round's
-    search, whose stage time is that one kernel."""
+    (k_seed_dists: it reads the n query rows and writes n*32 distances; with the relocation of the
+    base it is timed inside round 1's stage), so no search launch gathers a seed row.  The reported
+    launch is the last round's search, whose stage time is that one kernel."""
     n, d, L = args.n, args.d, args.beam
 
     def kernel_bytes(r):
@@ -257,7 +273,7 @@ def search_roofline(st, args, peak_gbs, peak_kind, rounds):
         out["round1_stage"] = {"algorithmic_bytes": int(b0), "ms": round(st.ms_search[0], 3),
                                "achieved": round(b0 / (st.ms_search[0] / 1e3) / 1e9, 1),
                                "traffic": dram[0] if dram else None,
-                               "includes": "seed pre-pass + round-1 search"}
+                               "includes": "seed pre-pass, relocation, round-1 search"}
     return out
 
 
@@ -468,11 +484,7 @@ def run_ours(args):
     proj = torch.empty((n, 16), dtype=torch.int32, device=dev)
     stream = torch.cuda.Stream(dev)
     h = pg.Handle(local, stream=stream)
-    # K0, K2 + CSR (5), K3 = 8; per link round search, prune + CSR (5), merge = 8; once per build
-    # the seed-distance pass and, when screened, the norm pre-pass
-    once = (1 if params.link_rounds > 0 else 0) + (
-        1 if (screen and params.link_rounds > 0 and args.beam <= 128) else 0)
-    launches_per_build = 8 + 8 * params.link_rounds + once
+    launches_per_build = build_launches(n, d, params)
     tuning = None
     if args.autotune:
         t0 = time.perf_counter()
@@ -787,7 +799,8 @@ def run_batched(args):
     with ClockSampler(0) as clocks:
         res, st, ms = batched_measure(h, stream, base, gt, node_off, sizes, args.degree,
                                       args.beam, screen, args.steps, args.warmup)
-    launches = (10 + 8 * 2 + 1 + (1 if screen and args.beam <= 128 else 0)) * args.steps
+    params = pg.default_params(args.degree, args.beam, screen=screen)
+    launches = build_launches(total, args.d, params, args.batched) * args.steps
     line = {"metric": metric_name(args, total), "value": st.evals_total / (ms / 1e3),
             "unit": UNIT, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": round(ms, 3), "higher_is_better": True, "scaling": "weak",

@@ -436,8 +436,8 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     pa.place = place;
     pa.norms = norms;
     PG_CUDA(pg::launch_prune_reverse(pa, true, sms, s));
-    PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->proj_pruned, n, indeg, offs, tsum, cursor, edges,
-                                   sms, s, 0, order, pdist));
+    PG_CUDA(pg::launch_reverse_csr(pruned, pnum, p->proj_pruned, n, indeg, offs, tsum, cursor,
+                                   edges, sms, s, 0, order, pdist));
     PG_CUDA(pg::launch_reverse_lists(offs, edges, n, p->proj_reverse, rev, rnum, sms, s, place,
                                      rdist));
     // K3 phase-1 merge -> projection graph
@@ -1397,7 +1397,7 @@ int pg_autotune(pg_handle h, pg_params* p, const float* d_base, uint32_t d, cons
       if (rc) return restore(rc);
     }
     if (tp.screen != PG_SCREEN_NONE) {
-      for (uint32_t c : {3u, 4u}) {
+      for (uint32_t c : {2u, 4u}) {
         rc = try_value(&pg_tuning::screen_stages, c);
         if (rc) return restore(rc);
       }

@@ -418,7 +418,8 @@ __device__ __forceinline__ void prune_node(const PruneArgs& a, NodeLists<W>* sm,
 constexpr int kPruneWarps = 24;  // warps per SM (80 registers)
 
 template <int W, bool PHASE1, bool SCREEN, bool WIDE>
-__global__ void __launch_bounds__(32 * W, kPruneWarps / W) k_prune_reverse(PruneArgs a, uint32_t look) {
+__global__ void __launch_bounds__(32 * W, kPruneWarps / W)
+k_prune_reverse(PruneArgs a, uint32_t look) {
   __shared__ NodeLists<W> sm;
   uint32_t part = 0;
   uint64_t ev = 0;
@@ -449,8 +450,8 @@ __global__ void __launch_bounds__(32 * W, kPruneWarps / W) k_prune_reverse(Prune
   if (lane_id() == 0 && ev) atomicAdd(a.evals, static_cast<unsigned long long>(ev));
 }
 
-// The distances of the screened prune's kept edges, which the merge sorts by: one edge per lane, the
-// edges of `look` nodes at a time (two or three a node on 1M x 200; at most 32).
+// The distances of the screened prune's kept edges, which the merge sorts by: one edge per lane,
+// the edges of `look` nodes at a time (two or three a node on 1M x 200; at most 32).
 template <bool WIDE>
 __global__ void __launch_bounds__(256) k_edge_dists(const float* __restrict__ base, uint64_t n,
                                                     uint32_t d,

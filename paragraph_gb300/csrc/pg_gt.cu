@@ -418,8 +418,8 @@ cudaError_t launch_final(const GtArgs& f, int num_sms, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// The k-th largest of the values that `each` visits, given the smallest (mn) and largest (mx) of them
-// and at least k of them; one warp.  A histogram of kThetaBins equal steps between the two finds
+// The k-th largest of the values that `each` visits, given the smallest (mn) and largest (mx) of
+// them and at least k of them; one warp.  A histogram of kThetaBins equal steps between the two finds
 // the step that holds it; that step's few values are then gathered and ranked.  A step with more
 // than kThetaBins of them (an outlier far above the rest) is divided again.  The values spread over
 // the steps, so the shared-memory counters see few collisions, and three passes over them mostly
@@ -510,9 +510,9 @@ __device__ float kth_largest(Each each, float mn, float mx, uint32_t k, uint32_t
   return mn;
 }
 
-// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima (-inf when
-// there are fewer than k groups: every base row is then a candidate).  3.4 -> 1.6 ms for 250k rows of
-// 4700 maxima against a radix select, whose first of four histograms collides on the sign and
+// One warp per query: lo = theta - 2 E_q, theta the k-th largest of the row's group maxima (-inf
+// when there are fewer than k groups: every base row is then a candidate).  3.4 -> 1.6 ms for 250k
+// rows of 4700 maxima against a radix select, whose first of four histograms collides on the sign and
 // exponent.
 template <bool PAIRS>  // an even number of groups: rows start on 8 bytes
 __global__ void __launch_bounds__(256) k_gt_theta(const float* __restrict__ maxima,

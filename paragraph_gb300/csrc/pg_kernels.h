@@ -35,8 +35,8 @@ struct PruneArgs {
   // depend on it
   uint32_t stages;
   uint32_t screen_half;  // screened kernel: FP16 operands instead of BF16
-  // screened builds: per point (|x|, |x - x^| + |x^_sub|) upper bounds (phase 1 too) and the 16-bit rows from
-  // launch_screen_norms with the same screen_half, and the candidates' distances (n x c) from
+  // screened builds: per point (|x|, |x - x^| + |x^_sub|) upper bounds (phase 1 too) and the 16-bit
+  // rows from launch_screen_norms with the same screen_half, and the candidates' distances (n x c) from
   // launch_list_dists
   const float2* norms;
   const void* rows16;
@@ -215,8 +215,8 @@ cudaError_t launch_reverse_csr(const uint32_t* pruned, const uint32_t* pruned_nu
                                int num_sms, cudaStream_t st, uint64_t rows = 0,
                                const uint32_t* order = nullptr,
                                const float* pruned_dist = nullptr);
-// indeg is left zero.  With pruned_dist / rev_dist every edge carries its distance (edges: 8 bytes each).
-// With order / place (relocated builds) the edges hold original ids, which decide which sources a
+// indeg is left zero.  With pruned_dist / rev_dist every edge carries its distance (edges: 8 bytes
+// each).  With order / place (relocated builds) the edges hold original ids, which decide which sources a
 // list keeps and their sequence, and the lists hold places.
 cudaError_t launch_reverse_lists(const uint32_t* offs, const uint32_t* edges, uint64_t n,
                                  uint32_t r, uint32_t* rev, uint32_t* rev_num, int num_sms,

@@ -16,8 +16,9 @@
 //      for the chunk: the Gram G = A A^T of the tile's 16-bit rows accumulates in 128 TMEM
 //      columns, and each node's block of G lies in the node's own TMEM lanes and columns;
 //   3. the distance of each candidate to the node comes from the search, which computed it in
-//      another FP32 order (launch_list_dists fills in the few it has not); the nearest undecided candidate is the one whose interval lies below
-//      the others', or the exact minimum (distance, slot) of those whose intervals overlap;
+//      another FP32 order (launch_list_dists fills in the few it has not); the nearest undecided
+//      candidate is the one whose interval lies below the others', or the exact minimum
+//      (distance, slot) of those whose intervals overlap;
 //   4. for each kept entry r every undecided candidate p reads G[p][r] from its own TMEM lane (one
 //      tcgen05.ld column) and decides dist(p, r) < d_p from it outside the bound, or by exact
 //      chains.  A candidate's recorded occluder is thus the first kept entry, in kept order, that
@@ -229,10 +230,10 @@ __device__ __forceinline__ void fma4(float4& s, const float4 u, const float4 v) 
 __device__ __forceinline__ float sum4(const float4 s) { return (s.x + s.y) + (s.z + s.w); }
 
 // FP32 inner products of row r with the rows x of the lanes that `want` one, each valid in its
-// lane.  Loads are whole 128-byte lines.  Four rows at a time, eight lanes each; with WHOLE the last
-// one or two take the whole warp, which holds a row of 512 floats in one round of loads.  That is
-// the usual case in the prune, whose scan waits for it: round 2 of 1M x 512 97.6 -> 87.0 ms, but of
-// 1M x 200 9.0 -> 9.5 (the larger kernel), hence only for rows over 256 floats.
+// lane.  Loads are whole 128-byte lines.  Four rows at a time, eight lanes each; with WHOLE the
+// last one or two take the whole warp, which holds a row of 512 floats in one round of loads.  That
+// is the usual case in the prune, whose scan waits for it: round 2 of 1M x 512 96.7 -> 87.7 ms, but
+// of 1M x 200 9.0 -> 9.5 (the larger kernel), hence only for rows over 256 floats.
 template <bool WHOLE>
 __device__ __forceinline__ float warp_dots(const float* __restrict__ base, uint32_t d, uint32_t r,
                                            uint32_t x, bool want) {

@@ -17,8 +17,8 @@
 //     order (the reference's one-thread order), through the same count/scan/scatter/sort CSR as
 //     the link rounds; a merged list too short to be pruned is written in ascending id order (the
 //     reference writes std::unordered_set order, which no consumer depends on).
-// Most lists are a few ids long and a few fill the capacity, so every stage runs twice: one warp per
-// node for lists of up to kShort ids, which also queues the longer ones, and one block per node
+// Most lists are a few ids long and a few fill the capacity, so every stage runs twice: one warp
+// per node for lists of up to kShort ids, which also queues the longer ones, and one block per node
 // over that queue.  With one warp per node for all lists and candidates tested four at a time, the
 // stages waited for the longest lists (about a millisecond each): 200k x 200, six MatchSup rounds
 // 33.7 -> 7.8 ms, FusionNN 8.2 -> 1.5, FusionFinal 7.0 -> 1.1.

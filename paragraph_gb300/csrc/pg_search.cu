@@ -665,11 +665,11 @@ cudaError_t launch_seed_dists(const SearchArgs& a, float* out, uint32_t* keys, u
 // neighbouring warps gather next to each other: fewer DRAM rows, fewer address translations, more
 // cache hits.  Nothing in the search or the prunes depends on the numbering (ties go by position);
 // the reverse lists, which keep the first sources by id, are sorted by original id.
-// Whole builds on the caller's rows -> relocated: 1M x 512 cosine (L = 96) 758 -> 491 ms, 300k x 512
-// 199 -> 147, 1M x 200 72.3 -> 69.5, 100k x 200 8.80 -> 8.53, 50k x 200 4.97 -> 4.81, 20k x 200
-// 2.53 -> 2.57, 10k x 512 4.33 -> 4.53: below 32 MB the base stays in L2 and the extra passes cost
-// more than they give.  The copy doubles the base's memory, so it stops at 32 GB (and where the
-// workspace cannot be allocated).
+// Whole builds on the caller's rows -> relocated: 1M x 512 cosine (L = 96) 758 -> 491 ms,
+// 300k x 512 199 -> 147, 1M x 200 72.3 -> 69.5, 100k x 200 8.80 -> 8.53, 50k x 200 4.97 -> 4.81,
+// 20k x 200 2.53 -> 2.57, 10k x 512 4.33 -> 4.53: below 32 MB the base stays in L2 and the extra
+// passes cost more than they give.  The copy doubles the base's memory, so it stops at 32 GB (and
+// where the workspace cannot be allocated).
 uint32_t reloc_keys(uint64_t n, uint32_t d, uint32_t seg_count) {
   constexpr uint64_t kMin = 32ull << 20, kMax = 32ull << 30;  // bytes of the base
   if (n * d * 4 < kMin || n * d * 4 > kMax || seg_count > 2048) return 0;

@@ -39,8 +39,10 @@
 // L2 gathers.  Streaming the FP32 rows instead, with the exact chain and the rounding of every
 // candidate done by its thread, and exact chains for every test inside the 16-bit margin, took
 // 10.6 + 10.7 ms at 1M x 200 and 22 + 31 ms at 300k x 512, L = 96.  Now 7.1 + 7.6 ms, with 0.5 ms
-// each for launch_list_dists and launch_edge_dists, and 17 + 29 ms with them.  Two or four stages
-// are 2-4% slower than three.
+// each for launch_list_dists and launch_edge_dists, and 15.8 + 26.9 ms with them.  Two or four
+// stages are 2-4% slower than three.  Putting a doubtful test off until its candidate may be kept
+// gained nothing (1M x 200 56.1 -> 57.6 ms, 1M x 512 335 -> 361): the next kept entry is usually
+// among the doubtful.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

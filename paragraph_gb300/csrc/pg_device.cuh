@@ -93,7 +93,6 @@ constexpr uint32_t kNoKey = 0xFFFFFFFFu;  // a list entry whose distance the sea
 __device__ __forceinline__ uint64_t pack_key(float dist, uint32_t pos) {
   return (static_cast<uint64_t>(order_key(dist)) << 32) | pos;
 }
-__device__ __forceinline__ uint32_t key_pos(uint64_t k) { return static_cast<uint32_t>(k); }
 
 // Warp bitonic sort of 32*E (key, value) pairs, ascending.  Element i lives in lane i % 32,
 // register slot i / 32.  Keys must be unique for a deterministic result (pack_key makes them so).

@@ -170,12 +170,16 @@ struct pg_handle_s {
 
 namespace {
 
+// A captured build holds addresses of the handle's buffers (workspace, sub-index table) and its launch
+// shapes: whatever changes one of them drops it.
+void drop_graph(pg_handle h) {
+  if (h->gexec) cudaGraphExecDestroy(h->gexec);
+  h->gexec = nullptr;
+}
+
 int ensure_ws(pg_handle h, size_t bytes) {
   if (bytes <= h->ws_bytes) return PG_OK;
-  if (h->gexec) {  // a captured build refers to the old workspace
-    cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-  }
+  drop_graph(h);
   if (h->ws) cudaFree(h->ws);
   h->ws = nullptr;
   h->ws_bytes = 0;
@@ -191,6 +195,7 @@ int ensure_ws(pg_handle h, size_t bytes) {
 
 int ensure_segs(pg_handle h, size_t words) {
   if (words <= h->segs_cap) return PG_OK;
+  drop_graph(h);  // it copies the old table
   if (h->h_segs) cudaFreeHost(h->h_segs);
   h->h_segs = nullptr;
   h->segs_cap = 0;
@@ -592,8 +597,7 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
     key.segs.assign(h->h_segs ? h->h_segs : nullptr,
                     h->h_segs ? h->h_segs + (seg_count ? 2 * (seg_count + 1) : 0) : nullptr);
     if (!h->gexec || !(h->gkey == key)) {
-      if (h->gexec) cudaGraphExecDestroy(h->gexec);
-      h->gexec = nullptr;
+      drop_graph(h);
       cudaGraph_t graph = nullptr;
       PG_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
       rc = enqueue();
@@ -1221,10 +1225,7 @@ int pg_set_tuning(pg_handle h, const pg_tuning* t) {
     return fail(PG_EINVAL, "screen_stages must be 0, 2, 3 or 4");
   std::lock_guard<std::mutex> lk(h->mu);
   h->tune = *t;
-  if (h->gexec) {  // a captured build holds the old launch shapes
-    cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-  }
+  drop_graph(h);
   return PG_OK;
 }
 
@@ -1405,10 +1406,7 @@ int pg_autotune(pg_handle h, pg_params* p, const float* d_base, uint32_t d, cons
   }
   best.ms_build = cur;
   h->tune = best;
-  if (h->gexec) {
-    cudaGraphExecDestroy(h->gexec);
-    h->gexec = nullptr;
-  }
+  drop_graph(h);
   p->km = tp.km;
   if (out) *out = best;
   return PG_OK;

@@ -93,7 +93,10 @@ struct NodeLists {
   uint64_t key[kCap];
   uint32_t id[kCap];    // sorted by (distance, position)
   float dist[kCap];
-  uint32_t kept[kCap];
+  // The scans keep at most the list's entries.  The merge's fill (not strict) then takes every entry
+  // not yet listed, where a kept id lists its first occurrence only: an id kept k times leaves k - 1 of
+  // its entries to be taken, so the two together stay below twice the list.
+  uint32_t kept[2 * kCap];
   uint8_t kpos[kCap];   // kept entries' places in the sorted list
   uint8_t own[kCap];    // entries known not to occlude one another (see merge_node)
   uint8_t und[kCap];    // undecided entries' places, ascending
@@ -733,6 +736,7 @@ template <int W, bool SCREEN, bool WIDE>
 __device__ __forceinline__ void merge_node(const MergeArgs& a, NodeLists<W>* sm, uint64_t b,
                                            uint32_t rn, uint32_t nn, uint64_t* ev) {
   using T = Team<W>;
+  static_assert(sizeof(sm->kept) >= 2 * 32 * W * sizeof(uint32_t), "kept entries and the fill's");
   const uint32_t t = T::tid(), lane = lane_id();
   const float* brow = a.base + b * a.d;
   uint32_t x = kTomb;

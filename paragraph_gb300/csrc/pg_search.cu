@@ -200,6 +200,12 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
   return (v[0] + v[2]) + (v[1] + v[3]);
 }
 
+// The lines of a row to L2, without waiting for them.
+__device__ __forceinline__ void prefetch_row(const float* row, uint32_t d) {
+  for (uint32_t c = 0; c < d; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(row + d - 1));  // a row that starts inside a line
+}
+
 // Distances of the lanes whose `newc` is set (FLT_MAX elsewhere), up to ROWS rows per pass.
 template <int KSTEPS, int ROWS, bool FEW>
 __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTEPS>& q,
@@ -209,6 +215,10 @@ __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTE
   const uint32_t nnew = __popc(newmask);
   const uint32_t ci = __popc(newmask & ((1u << lane) - 1u));
   if (newc) list[ci] = node;
+  if constexpr (FEW && KSTEPS > 8) {  // the rows of the later passes, which wait for each other
+    if (a.prefetch && newc && ci >= ROWS)
+      prefetch_row(a.base + static_cast<uint64_t>(node) * a.d, a.d);
+  }
   __syncwarp();
   float result = FLT_MAX;
   for (uint32_t c0 = 0; c0 < nnew; c0 += ROWS) {
@@ -785,10 +795,18 @@ cudaError_t launch_search(const SearchArgs& a, int num_sms, size_t smem_optin, c
   // against 152 us; 1216: 125 against 103).
   const uint64_t nq = a.queries ? a.nq : a.n;
   const bool few = nq <= static_cast<uint64_t>(num_sms) * 8 || (a.rows == 16 && a.km == 32);
+  // Few long rows: the passes of an iteration wait for each other, so rows that lie in DRAM (queries
+  // not asked before) cost one DRAM latency per pass.  Sending the later passes' rows to L2 first pays
+  // there and costs a little on rows already in L2.  16 queries x 512, Km = 32, L2 flushed 224 -> 209
+  // us, asked again 183 -> 184; 16 x 384, Km = 96, 495 -> 449 and 296 -> 308.  Up to 320 floats it
+  // cost as much as it gave (260: 139 -> 132 and 110 -> 113), and with more than two queries per SM
+  // other queries hide the latency (1000 x 512: 300 -> 302 and, 400k points, 125 -> 134).
+  SearchArgs b = a;
+  b.prefetch = a.d > 320 && nq <= static_cast<uint64_t>(num_sms) * 2;
   switch (a.km / 32) {
-    case 1: return launch_search_d<1>(a, few, num_sms, smem_optin, st);
-    case 2: return launch_search_d<2>(a, few, num_sms, smem_optin, st);
-    default: return launch_search_d<3>(a, few, num_sms, smem_optin, st);
+    case 1: return launch_search_d<1>(b, few, num_sms, smem_optin, st);
+    case 2: return launch_search_d<2>(b, few, num_sms, smem_optin, st);
+    default: return launch_search_d<3>(b, few, num_sms, smem_optin, st);
   }
 }
 

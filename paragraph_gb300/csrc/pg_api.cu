@@ -1282,7 +1282,7 @@ int pg_autotune(pg_handle h, pg_params* p, const float* d_base, uint32_t d, cons
   pg_tuning best{};
   best.search_rows = 8;
   best.hash_factor = 1;
-  best.screen_stages = 2;
+  best.screen_stages = pg::kPruneStages;
   h->tune = best;
   pg_stats st;
 

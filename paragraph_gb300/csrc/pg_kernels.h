@@ -31,7 +31,7 @@ struct PruneArgs {
   uint32_t seg_count;
   // relocated builds: place of every original id (phase 1 reads original ids from gt), else NULL
   const uint32_t* place;
-  // screened kernel: depth of its row-copy ring (0 = default, else 2..4); results do not
+  // screened kernel: depth of its row-copy ring (0 = kPruneStages, else 2..4); results do not
   // depend on it
   uint32_t stages;
   uint32_t screen_half;  // screened kernel: FP16 operands instead of BF16
@@ -248,6 +248,7 @@ cudaError_t launch_reloc_rows(const float* base, uint64_t n, uint32_t d, const f
                               const uint32_t* order, float* out_base, float* out_seeds,
                               int num_sms, cudaStream_t st);
 bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd);
+constexpr uint32_t kPruneStages = 3;  // default depth of the screened prune's copy ring
 // Screened prune for strict rounds (pg_prune_tc.cu): FP16 or BF16 candidate Gram on the tcgen05
 // tensor cores + exact re-scoring, 1 <= c <= 128, 4 <= d <= 1024, d % 4 == 0; the launch also
 // wants a 16-byte aligned base.

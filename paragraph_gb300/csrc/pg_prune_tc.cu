@@ -88,7 +88,7 @@ __host__ __device__ constexpr Layout layout(uint32_t stages) {
   l.total = l.words + 16;
   return l;
 }
-constexpr uint32_t kMinStages = 2, kMaxStages = 4, kDefaultStages = 3;
+constexpr uint32_t kMinStages = 2, kMaxStages = 4;
 size_t smem_bytes(uint32_t stages) { return layout(stages).total + 1024; }
 
 // 16 bytes global -> shared, cached in L2 only, completing with the thread's copy groups.
@@ -670,7 +670,7 @@ cudaError_t launch_prune_screen(const PruneArgs& a, int num_sms, size_t smem_opt
   sh.nk = (sh.dp + kCk - 1) / kCk;
   const uint32_t per_tile = kTile / sh.cap;
   sh.tiles = (a.n + per_tile - 1) / per_tile;
-  uint32_t s = a.stages ? a.stages : kDefaultStages;
+  uint32_t s = a.stages ? a.stages : kPruneStages;
   if (s < kMinStages) s = kMinStages;
   if (s > kMaxStages) s = kMaxStages;
   while (s > kMinStages && smem_bytes(s) > smem_optin) s--;

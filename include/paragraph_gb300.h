@@ -126,9 +126,11 @@ int pg_params_default(pg_params* p, uint32_t degree, uint32_t beam);
  * cudaStream_t (NULL = the legacy default stream).  One build in flight per handle. */
 int pg_create(pg_handle* out, int device, void* stream);
 int pg_destroy(pg_handle h);
-/* Device bytes the handle allocates for a build of n points (the caller can check headroom).  For a
- * base of 32 MB to 32 GB this includes a sorted copy of it; where that cannot be allocated the build
- * works on the caller's rows instead, slower and with the same result. */
+/* Device bytes the handle allocates for a build of n points where they are free (the caller can
+ * check headroom).  For a base of 32 MB to 32 GB this includes a sorted copy of it.  A build that
+ * finds less works without the copy, and with less still without the tensor-core prune and the
+ * stored distances: slower, with the same result, in as little as a third of these bytes.  It looks
+ * again on each call. */
 int pg_workspace_bytes(const pg_params* p, uint64_t n, uint32_t d, uint64_t q, uint64_t* bytes);
 
 /* ---- whole build (Gbuilder::Builder<float>::LaunchBuild, include/Builder.hpp:15-35) ------- */

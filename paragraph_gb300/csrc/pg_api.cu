@@ -50,32 +50,24 @@ enum Counter {
   C_COUNT = 22
 };
 
-struct Workspace {
-  uint32_t* winner = nullptr;
-  uint32_t* pruned = nullptr;
-  uint32_t* pruned_num = nullptr;
-  uint32_t* indeg = nullptr;
-  uint32_t* offs = nullptr;
-  uint32_t* tile_sums = nullptr;
-  uint32_t* cursor = nullptr;
-  uint32_t* edges = nullptr;
-  uint32_t* rev = nullptr;
-  uint32_t* rev_num = nullptr;
-  uint32_t* sres = nullptr;
-  uint32_t* proj = nullptr;
-  uint32_t* graph = nullptr;
-};
-
 size_t align_up(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 struct Layout {
   size_t winner, pruned, pruned_num, indeg, offs, tile_sums, cursor, edges, rev, rev_num, sres,
-      proj, graph, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place,
+      proj, segs, norms, seeds, rbase, rseeds, rproj, rgraph, keys, bins, order, place,
       pruned_dist, rev_dist, queue, rows16, sdist, total;
 };
 
+// How a build is laid out.  Every choice gives the same result.
+struct BuildPlan {
+  uint32_t nkeys;  // locality keys of the sorted copy of the base; 0: work on the caller's rows
+  bool carry;      // lists and edges carry their distances, else the merges compute them again
+  bool screened;   // prunes on the tensor cores (needs carry)
+};
+
+// own_proj: a place for the projection, which otherwise goes straight to the caller's buffer.
 Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_t L,
-                   uint32_t proj_deg, uint32_t degree, uint32_t nkeys, bool screened,
+                   uint32_t proj_deg, uint32_t degree, const BuildPlan& plan, bool own_proj,
                    uint32_t seg_count = 0) {
   Layout l{};
   size_t o = 0;
@@ -91,31 +83,34 @@ Layout make_layout(uint64_t n, uint32_t d, uint32_t pmax, uint32_t rmax, uint32_
   l.offs = take((n + 1) * 4);
   l.tile_sums = take(((n + pg::kScanTileElems - 1) / pg::kScanTileElems + 1) * 4);
   l.cursor = take(n * 4);
-  l.edges = take(n * pmax * 8);
+  l.edges = take(n * pmax * (plan.carry ? 8 : 4));
   l.rev = take(n * rmax * 4);
   l.rev_num = take(n * 4);
-  l.pruned_dist = take(n * pmax * 4);
-  l.rev_dist = take(n * rmax * 4);
+  if (plan.carry) {
+    l.pruned_dist = take(n * pmax * 4);
+    l.rev_dist = take(n * rmax * 4);
+  }
   l.queue = take((n + 2) * 4);
   l.sres = take(n * L * 4);
-  l.proj = take(n * proj_deg * 4);
-  l.graph = take(n * degree * 4);
+  if (own_proj && !plan.nkeys) l.proj = take(n * proj_deg * 4);
   l.segs = take(2 * (static_cast<size_t>(seg_count) + 1) * 8);
-  if (screened) {  // screened prune: per-point norm bounds, 16-bit rows, the lists' distances
+  if (plan.screened) {  // per-point norm bounds, 16-bit rows, the lists' distances
     l.norms = take(n * 8);
     l.rows16 = take(n * pg::screen_row(d) * 2);
     l.sdist = take(n * L * 4);
   }
-  l.seeds = take(n * 32 * 4);  // link-round searches: every query's 32 seed distances
-  if (nkeys) {  // relocated build: the sorted copy of the base, seed distances and graphs by place
+  if (plan.nkeys) {  // the sorted copy of the base, seed distances and graphs by place
+    l.seeds = l.sres;  // copied to rseeds before the first search (L >= 64 in relocated builds)
     l.rbase = take(n * d * 4);
     l.rseeds = take(n * 32 * 4);
     l.rproj = take(n * proj_deg * 4);
     l.rgraph = take(n * degree * 4);
     l.keys = take(n * 4);
-    l.bins = take(nkeys * 4);
+    l.bins = take(plan.nkeys * 4);
     l.order = take(n * 4);
     l.place = take(n * 4);
+  } else {
+    l.seeds = take(n * 32 * 4);  // link-round searches: every query's 32 seed distances
   }
   l.total = o;
   return l;
@@ -146,7 +141,6 @@ struct pg_handle_s {
   size_t smem_optin = 0;
   char* ws = nullptr;
   size_t ws_bytes = 0;
-  size_t reloc_limit = ~static_cast<size_t>(0);  // a relocated build's workspace did not fit
   char* inbuf = nullptr;  // device copies of host inputs (pg_build_host)
   size_t in_bytes = 0;
   uint32_t* d_status = nullptr;
@@ -177,12 +171,28 @@ void drop_graph(pg_handle h) {
   h->gexec = nullptr;
 }
 
-int ensure_ws(pg_handle h, size_t bytes) {
-  if (bytes <= h->ws_bytes) return PG_OK;
+void release_ws(pg_handle h) {
   drop_graph(h);
   if (h->ws) cudaFree(h->ws);
   h->ws = nullptr;
   h->ws_bytes = 0;
+}
+
+// Whether a workspace of this size is there or could be allocated now.  Asked before a build gives up
+// the workspace it has for a larger one that it can do without.
+bool room_for_ws(pg_handle h, size_t bytes) {
+  if (bytes <= h->ws_bytes) return true;
+  size_t avail = 0, all = 0;
+  if (cudaMemGetInfo(&avail, &all) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return bytes <= avail + h->ws_bytes;
+}
+
+int ensure_ws(pg_handle h, size_t bytes) {
+  if (bytes <= h->ws_bytes) return PG_OK;
+  release_ws(h);
   cudaError_t e = cudaMalloc(&h->ws, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -191,6 +201,18 @@ int ensure_ws(pg_handle h, size_t bytes) {
   }
   h->ws_bytes = bytes;
   return PG_OK;
+}
+
+// Memory of a call that has not begun to use the workspace.  An earlier build's workspace may hold more
+// than that build needed: it makes room, and the call takes another.
+cudaError_t malloc_beside_ws(pg_handle h, char** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && h->ws) {
+    cudaGetLastError();
+    release_ws(h);
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
 }
 
 int ensure_segs(pg_handle h, size_t words) {
@@ -213,7 +235,7 @@ int ensure_in(pg_handle h, size_t bytes) {
   if (h->inbuf) cudaFree(h->inbuf);
   h->inbuf = nullptr;
   h->in_bytes = 0;
-  cudaError_t e = cudaMalloc(&h->inbuf, bytes);
+  cudaError_t e = malloc_beside_ws(h, &h->inbuf, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(PG_ENOMEM, "cudaMalloc of %zu input bytes failed: %s", bytes,
@@ -311,25 +333,26 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   const uint32_t L = p->km + p->kp * p->kd;
   const uint32_t pmax = std::max(p->proj_pruned, p->degree);
   const uint32_t rmax = std::max(p->proj_reverse, p->link_reverse);
-  const bool screened = p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1);
-  uint32_t nkeys = p->link_rounds ? pg::reloc_keys(n, d, seg_count) : 0;
-  auto shape = [&]() {
-    return make_layout(n, d, pmax, rmax, L, p->proj_degree, p->degree, nkeys, screened,
-                       seg_count);
-  };
-  Layout lay = shape();
-  if (nkeys && lay.total >= h->reloc_limit) {
-    nkeys = 0;
-    lay = shape();
-  }
-  int rc = ensure_ws(h, lay.total);
-  if (rc == PG_ENOMEM && nkeys) {  // no room for the copy: build on the caller's rows
-    h->reloc_limit = lay.total;
-    nkeys = 0;
-    lay = shape();
+  // The fastest plan whose workspace can be had: on a sorted copy of the base, on the caller's rows, or
+  // without what only saves time (3.5, 2.5 and 1.1 KB per point of 200 floats, M = 32, L = 64).
+  const bool screen = p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1);
+  const BuildPlan plans[] = {{p->link_rounds ? pg::reloc_keys(n, d, seg_count) : 0, true, screen},
+                             {0, true, screen},
+                             {0, false, false}};
+  BuildPlan plan{};
+  Layout lay{};
+  int rc = PG_ENOMEM;
+  for (size_t i = 0; i < 3 && rc == PG_ENOMEM; i++) {
+    plan = plans[i];
+    if (i == 0 && !plan.nkeys) continue;
+    lay = make_layout(n, d, pmax, rmax, L, p->proj_degree, p->degree, plan, proj_out == nullptr,
+                      seg_count);
+    if (i < 2 && !room_for_ws(h, lay.total)) continue;
     rc = ensure_ws(h, lay.total);
   }
   if (rc) return rc;
+  const uint32_t nkeys = plan.nkeys;
+  const bool screened = plan.screened;
   char* w = h->ws;
   uint32_t* winner = reinterpret_cast<uint32_t*>(w + lay.winner);
   uint32_t* pruned = reinterpret_cast<uint32_t*>(w + lay.pruned);
@@ -341,8 +364,8 @@ int run_build(pg_handle h, const pg_params* p, const float* base, uint64_t n, ui
   uint32_t* edges = reinterpret_cast<uint32_t*>(w + lay.edges);
   uint32_t* rev = reinterpret_cast<uint32_t*>(w + lay.rev);
   uint32_t* rnum = reinterpret_cast<uint32_t*>(w + lay.rev_num);
-  float* pdist = reinterpret_cast<float*>(w + lay.pruned_dist);
-  float* rdist = reinterpret_cast<float*>(w + lay.rev_dist);
+  float* pdist = plan.carry ? reinterpret_cast<float*>(w + lay.pruned_dist) : nullptr;
+  float* rdist = plan.carry ? reinterpret_cast<float*>(w + lay.rev_dist) : nullptr;
   uint32_t* queue = reinterpret_cast<uint32_t*>(w + lay.queue);
   uint32_t* sres = reinterpret_cast<uint32_t*>(w + lay.sres);
   uint32_t* proj = nkeys ? reinterpret_cast<uint32_t*>(w + lay.rproj)
@@ -665,7 +688,7 @@ int ensure_ws2(pg_handle h, size_t bytes) {
   if (h->ws2) cudaFree(h->ws2);
   h->ws2 = nullptr;
   h->ws2_bytes = 0;
-  cudaError_t e = cudaMalloc(&h->ws2, bytes);
+  cudaError_t e = malloc_beside_ws(h, &h->ws2, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(PG_ENOMEM, "cudaMalloc of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
@@ -917,10 +940,11 @@ int pg_workspace_bytes(const pg_params* p, uint64_t n, uint32_t d, uint64_t q, u
   if (rc) return rc;
   if (!bytes) return fail(PG_EINVAL, "bytes is NULL");
   const uint32_t L = p->km + p->kp * p->kd;
+  const BuildPlan plan{p->link_rounds ? pg::reloc_keys(n, d, 0) : 0, true,
+                       p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1)};
   Layout l = make_layout(n, d, std::max(p->proj_pruned, p->degree),
                          std::max(p->proj_reverse, p->link_reverse), L, p->proj_degree, p->degree,
-                         p->link_rounds ? pg::reloc_keys(n, d, 0) : 0,
-                         p->screen != PG_SCREEN_NONE && pg::screen_supported(L, d, 1));
+                         plan, true);
   *bytes = l.total;
   return PG_OK;
 }

@@ -1688,7 +1688,7 @@ int pg_ground_truth(pg_handle h, const float* d_base, uint64_t n, uint32_t d,
     PG_CUDA(cudaMemcpyAsync(h->h_counters + 60, diag, 12, cudaMemcpyDeviceToHost, h->stream));
     PG_CUDA(cudaStreamSynchronize(h->stream));
     st = *h->h_status;
-    // a sampled threshold let too many candidates through: once more with every tile
+    // a sampled threshold still lets too many candidates through: once more with every tile
     if (plan.step == 1 || st != (1u << 6)) break;
   }
   const float* dg = reinterpret_cast<const float*>(h->h_counters + 60);

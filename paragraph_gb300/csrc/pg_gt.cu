@@ -25,8 +25,11 @@
 // With groups many enough that the top k fall in nearly distinct groups, theta_q sits just
 // below t_k and a query keeps about 1.1 k candidates.  From a sample of every step-th tile it keeps
 // about 1.1 k step, which k_gt_narrow brings back to 1.1 k; pass 1 then costs 1 / step of pass 2.
-// Data on which a sampled threshold lets through more than the selection holds (near rows placed to
-// miss the sample) are done again with every tile.
+// A query whose sampled threshold lets through more than its list holds (near rows that miss the
+// sample, as in a base stored cluster by cluster) is filtered again, up to twice: the k-th best of the
+// candidates that its list did hold is a higher threshold.  300k x 200 in the order of 1000 clusters,
+// 100k queries near them, k = 10: 47 ms (66 ms when one such query had the whole call done again with
+// every tile); shuffled 14.5 ms.  The two passes cost 20 us where there is nothing to do.
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -41,6 +44,8 @@ namespace pg {
 namespace {
 
 constexpr uint32_t kGtCap = 1024;          // candidates per query
+constexpr uint32_t kGtTile = 128;          // queries per tile of the GEMM passes
+constexpr int kGtAgain = 2;                // further filter passes after a sampled threshold
 constexpr uint32_t kGtErrRange = 1u << 4;  // a value beyond the FP16 range
 constexpr uint32_t kGtErrFinal = 1u << 6;  // a query kept more candidates than kGtCap
 constexpr uint32_t kGtShort = 256;         // lists of the final pass's common kernel
@@ -567,10 +572,15 @@ __global__ void __launch_bounds__(256) k_gt_theta(const float* __restrict__ maxi
 
 // After a sampled threshold: one warp per query keeps, of its candidates, those within 2 E_q of the
 // k-th largest screened score (all of them when there are no more than k), in the list's first half
-// and then its second.
+// and then its second.  A query with more candidates than its list holds takes that bound, from those
+// it does hold, as its threshold of another filter pass (`again` marks its tile of 128 queries); the
+// others' thresholds become infinite, so that pass leaves them alone.  first: of the passes; the later
+// ones look at the queries that were filtered again.  again == NULL: no pass follows.
 __global__ void __launch_bounds__(128) k_gt_narrow(uint64_t* __restrict__ cand,
                                                    uint32_t* __restrict__ cand_cnt, uint32_t rows,
-                                                   uint32_t k, const float* __restrict__ band) {
+                                                   uint32_t k, const float* __restrict__ band,
+                                                   float* __restrict__ lo,
+                                                   uint32_t* __restrict__ again, bool first) {
   __shared__ uint64_t buf_all[4][kGtCap];
   __shared__ uint32_t hist_all[4][kThetaBins];
   __shared__ uint32_t fill_all[4];
@@ -578,9 +588,12 @@ __global__ void __launch_bounds__(128) k_gt_narrow(uint64_t* __restrict__ cand,
   uint64_t* buf = buf_all[warp];
   const uint64_t nw = static_cast<uint64_t>(gridDim.x) * 4;
   for (uint64_t row = blockIdx.x * 4ull + warp; row < rows; row += nw) {
-    const uint32_t c0 = min(cand_cnt[2 * row], kGtCap / 2);
-    const uint32_t c1 = min(cand_cnt[2 * row + 1], kGtCap / 2);
+    if (!first && !(lo[row] < INFINITY)) continue;
+    const uint32_t n0 = cand_cnt[2 * row], n1 = cand_cnt[2 * row + 1];
+    const uint32_t c0 = min(n0, kGtCap / 2), c1 = min(n1, kGtCap / 2);
     const uint32_t cnt = c0 + c1;
+    const bool more = again && cnt < n0 + n1;
+    if (!more && lane == 0) lo[row] = INFINITY;
     if (cnt <= k) continue;
     uint64_t* list = cand + row * kGtCap;
     float mn = INFINITY, mx = -INFINITY;
@@ -600,6 +613,14 @@ __global__ void __launch_bounds__(128) k_gt_narrow(uint64_t* __restrict__ cand,
       for (uint32_t i = lane; i < cnt; i += 32) use(key_value(buf[i]));
     };
     const float low = kth_largest(each, mn, mx, k, hist_all[warp], fill_all + warp) - band[row];
+    if (more) {
+      if (lane == 0) {
+        lo[row] = fmaxf(lo[row], low);
+        again[row / kGtTile] = 1;
+      }
+      __syncwarp();
+      continue;
+    }
     uint32_t kept = 0;
     for (uint32_t i0 = 0; i0 < cnt; i0 += 32) {
       const uint32_t i = i0 + lane;
@@ -670,7 +691,11 @@ struct Args {
   float* maxima;    // kMax: nq x groups
   const float* lo;  // kFilter: nq thresholds
   uint64_t* cand;   // kFilter: nq x kGtCap keys, two halves of kGtCap / 2
-  uint32_t* cand_cnt;  // kFilter: nq x 2 (one count per half)
+  uint32_t* cand_cnt;  // kFilter: nq x 2 (hits per half, also those past the list's end)
+  // kFilter: the second pass after a sampled threshold sweeps the query tiles marked here, for their
+  // rows with a finite threshold; NULL: every tile and row
+  const uint32_t* again;
+  bool refuse;  // kFilter: no pass follows that could bring a list past its end back
   float* dump;      // kDump: nq x n scores
   uint32_t* status;
 };
@@ -731,6 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t q_tiles = (a.nq + rows_per_tile - 1) / rows_per_tile;
   const uint32_t n_tiles = ((a.n + BN - 1) / BN + a.step - 1) / a.step;  // tiles swept
   constexpr uint32_t ncols = 2 * BN * MT;  // two accumulator buffers per M tile (512)
+  auto swept = [&](uint32_t st) { return MODE != kFilter || !a.again || a.again[st] != 0; };
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < a.stages; s++) {
@@ -765,8 +791,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       bool ok = true;
       uint32_t it = 0, sti = 0;
-      for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x, sti++) {
-        if (!bar_wait(a_empty, (sti & 1u) ^ 1u, stop)) {
+      for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x) {
+        if (!swept(st)) continue;
+        const uint32_t sp = sti++ & 1u;
+        if (!bar_wait(a_empty, sp ^ 1u, stop)) {
           ok = false;
           break;
         }
@@ -805,8 +833,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool ok = true;
       uint32_t it = 0, t = 0, sti = 0;
       const uint32_t a0 = saddr(sA), b0 = saddr(sB);
-      for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x, sti++) {
-        if (!bar_wait(a_full, sti & 1u, stop)) {
+      for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x) {
+        if (!swept(st)) continue;
+        const uint32_t sp = sti++ & 1u;
+        if (!bar_wait(a_full, sp, stop)) {
           ok = false;
           break;
         }
@@ -844,8 +874,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         raise_error(a.status, kErrWait);
         *stop = 1;
       }
-      commit(drained);  // arrives when every MMA issued above has completed
-      bar_wait(drained, 0, nullptr);
+      if (sti) {
+        commit(drained);  // arrives when every MMA issued above has completed
+        bar_wait(drained, 0, nullptr);
+      }
     }
   } else {
     // ---- epilogue: one thread per (query row, half of the tile's columns)
@@ -857,6 +889,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t t = 0;
     const uint32_t chunks = n_tiles * kCpt;  // this thread's 32-column chunks per M tile
     for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x) {
+      if (!swept(st)) continue;
       uint32_t qrow[MT], cnt[MT];
       bool valid[MT];
       float lo[MT], run[MT];
@@ -865,6 +898,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         qrow[m] = st * rows_per_tile + m * kRows + row;
         valid[m] = qrow[m] < a.nq;
         lo[m] = (MODE == kFilter && valid[m]) ? a.lo[qrow[m]] : INFINITY;
+        if (MODE == kFilter && a.again) valid[m] = lo[m] < INFINITY;
         run[m] = -INFINITY;
         cnt[m] = 0;
       }
@@ -932,9 +966,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 1
               while (hit) {
                 const uint32_t j = static_cast<uint32_t>(__ffs(static_cast<int>(hit)) - 1);
-                hit &= hit - 1u;
-                if (cnt[m] < kHalfCap) dst[cnt[m]] = desc_key(tmp[j], col0 + j);
-                cnt[m]++;
+                const uint32_t c = cnt[m];
+                uint32_t at = c, pop = 1;
+                if (c < kHalfCap) {
+                  hit &= hit - 1u;
+                } else {  // past its end the list stays a sample of the hits, whose k-th best is then
+                          // worth most as the next threshold: one of these may take a place
+                  pop = __popc(hit);
+                  at = __umulhi(c * 0x9E3779B1u, c + pop) / pop;
+                  hit = 0;
+                }
+                if (at < kHalfCap) dst[at] = desc_key(tmp[j], col0 + j);
+                cnt[m] = c + pop;
               }
             }
           } else {
@@ -950,8 +993,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (uint32_t m = 0; m < MT; m++)
           if (valid[m]) {
-            a.cand_cnt[static_cast<uint64_t>(qrow[m]) * 2 + half] = min(cnt[m], kHalfCap);
-            if (cnt[m] > kHalfCap) raise_error(a.status, kGtErrFinal);
+            a.cand_cnt[static_cast<uint64_t>(qrow[m]) * 2 + half] = cnt[m];
+            if (cnt[m] > kHalfCap && a.refuse) raise_error(a.status, kGtErrFinal);
           }
       }
     }
@@ -1010,6 +1053,7 @@ cudaError_t launch_bn(const CUtensorMap& ta, const CUtensorMap& tb, const Args& 
 // The launched shape: 256 base rows per tile against one 128-row query tile (measured faster
 // than 128 base rows against two query tiles: 1.12 s against 1.28 s for 1M x 1M x 200).
 constexpr uint32_t kBN = 256;
+static_assert(kRows * (256 / kBN) == kGtTile, "query rows per tile");
 
 template <int MODE>
 cudaError_t launch(const CUtensorMap& ta, const CUtensorMap& tb, const Args& a, int num_sms,
@@ -1082,7 +1126,8 @@ GtPlan gt_plan(uint64_t n, uint64_t nq, uint32_t d, uint32_t k, bool sampled, in
 size_t gt_workspace_bytes(const GtPlan& p, uint64_t n, uint64_t nq) {
   auto al = [](uint64_t b) { return (b + 1023) & ~1023ull; };
   return al(n * p.dp * 2) + al(nq * p.dp * 2) + 2 * al(n * 4) + 2 * al(nq * 4) + al(8) +
-         2 * al(p.cq * 4) + al(p.cq * p.groups * 4) + al(p.cq * kGtCap * 8) + al(p.cq * 8);
+         2 * al(p.cq * 4) + al(p.cq * p.groups * 4) + al(p.cq * kGtCap * 8) + al(p.cq * 8) +
+         al((p.cq + kGtTile - 1) / kGtTile * 4);
 }
 
 int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
@@ -1109,6 +1154,8 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
   float* maxima = reinterpret_cast<float*>(take(cq * plan.groups * 4));
   uint64_t* cand = reinterpret_cast<uint64_t*>(take(cq * kGtCap * 8));
   uint32_t* cand_cnt = reinterpret_cast<uint32_t*>(take(cq * 8));
+  const uint64_t again_bytes = (cq + kGtTile - 1) / kGtTile * 4;
+  uint32_t* again = reinterpret_cast<uint32_t*>(take(again_bytes));
 
   cudaError_t e;
   k_half_rows<<<blocks_for(n, 8, num_sms, 8), 256, 0, st>>>(base, n, d, dp, b16, bn, be, status);
@@ -1147,10 +1194,22 @@ int ground_truth(const GtPlan& plan, const float* base, uint64_t n, uint32_t d,
     auto theta = plan.groups % 2 ? k_gt_theta<false> : k_gt_theta<true>;
     theta<<<blocks_for(rows, 8, num_sms, 8), 256, 0, st>>>(maxima, rows, plan.groups, k, band, lo);
     a.step = 1;
+    a.refuse = plan.step == 1;
     if ((e = tc::launch<tc::kFilter>(ta, tb, a, num_sms, st)) != cudaSuccess)
       return -static_cast<int>(e);
-    if (plan.step > 1)
-      k_gt_narrow<<<blocks_for(rows, 4, num_sms, 12), 128, 0, st>>>(cand, cand_cnt, rows, k, band);
+    if (plan.step > 1) {
+      const int blocks = blocks_for(rows, 4, num_sms, 12);
+      for (int pass = 0; pass < kGtAgain; pass++) {
+        if ((e = cudaMemsetAsync(again, 0, again_bytes, st)) != cudaSuccess)
+          return -static_cast<int>(e);
+        k_gt_narrow<<<blocks, 128, 0, st>>>(cand, cand_cnt, rows, k, band, lo, again, pass == 0);
+        a.again = again;
+        a.refuse = pass + 1 == kGtAgain;
+        if ((e = tc::launch<tc::kFilter>(ta, tb, a, num_sms, st)) != cudaSuccess)
+          return -static_cast<int>(e);
+      }
+      k_gt_narrow<<<blocks, 128, 0, st>>>(cand, cand_cnt, rows, k, band, lo, nullptr, false);
+    }
     GtArgs f{};
     f.base = base;
     f.queries = queries + q0 * d;

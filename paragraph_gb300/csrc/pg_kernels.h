@@ -98,7 +98,7 @@ struct SearchArgs {
   // same values the search would compute); NULL = the search scores the seeds itself
   const float* seed_dist;
   const uint32_t* place;  // relocated builds: place of every original id (the seeds), else NULL
-  uint32_t prefetch;  // set by launch_search: kernels for few queries send later rows to L2 ahead
+  uint32_t prefetch;  // set by launch_search: kernels for few queries send rows to L2 a pass ahead
 };
 
 // CPU RoarGraph path on the GPU (tests/test_t2iend.cu:365-613), pg_roar.cu.

@@ -51,7 +51,7 @@ __device__ __forceinline__ bool hash_test_and_set(uint32_t* t, uint32_t mask, ui
     if (old == key + 1) return false;
     s = (s + 1) & mask;
   }
-  return false;  // cannot happen: the table has twice the slots of the ids it ever holds
+  return false;  // cannot happen: the table has at least 1.6 times the slots of the ids it ever holds
 }
 
 __device__ __forceinline__ void hash_clear(uint32_t* t, uint32_t slots) {
@@ -112,15 +112,52 @@ struct Query {
   }
 };
 
+// How many queries a launch has for each SM, which decides how many registers a warp may take for
+// rows in flight.  A call with few queries lasts as long as its longest chain of row reads, so a warp
+// that shares its SM with few others takes more of them.
+enum class Load : int { kMany, kMid, kMidLong, kFew };
+
+// Rows per pass.  kMany: eight short rows (up to 256 floats) whole in flight, four long ones with
+// half of each in flight, or four where eight would spill (short rows past 224 floats, Km > 32: 3745
+// -> 2711 us for 39k queries, Km = 64).  Long rows, eight at a time with a quarter in flight: 4864
+// queries x 512, Km = 64: 1518 -> 1054 us, and 300k x 512 builds' searches 19.7 + 30.9 -> 16.9 + 27.7
+// ms.  kFew: 16 short or 8 long rows whole in flight (608 queries x 512, Km = 64: 601 -> 411 us).
+// Between them eight: whole, or long ones halved where sixteen warps share an SM.
+constexpr int search_rows(int km_s, int ksteps, Load load) {
+  if (load == Load::kFew) return ksteps > 8 ? 8 : 16;
+  if (load != Load::kMany) return 8;
+  return ksteps > 8 || (ksteps == 8 && km_s > 1) ? 4 : 8;
+}
+
+// Steps of 32 floats whose loads are in flight together.
+constexpr int load_steps(int ksteps, Load load) {
+  return ksteps > 8 && (load == Load::kMany || load == Load::kMid) ? 8 : ksteps;
+}
+
+// Warps per SM that the registers are allocated for.  kMany: the fastest of 16..32; one more or less
+// costs 1-3%, 16 or 32 cost 10-30% (too few warps, or spills).  The others hold one resident round of
+// the launches that take them.
+constexpr int search_warps(int km_s, int ksteps, Load load) {
+  if (load == Load::kFew) return 8;
+  if (load == Load::kMidLong) return 12;
+  if (load == Load::kMid) return 16;
+  return ksteps > 8 ? 24 : km_s == 1 ? 23 : ksteps == 8 ? 20 : 21;
+}
+
+// The lines of a row to L2, without waiting for them.
+__device__ __forceinline__ void prefetch_l2(const float* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Scores rows list[c0 .. c0 + 4R) (R rounds of four rows, one per 8-lane group; entries past the
 // last repeat it).  Lane (g, m) accumulates residues 4m..4m+3 of rows c0 + 4r + g (the
 // reference's lane-strided FMA chains), straight from global memory: one warp-wide load reads
 // four 128-byte row segments.  The first log2(R) butterfly levels are transposed (each lane keeps
 // one row), the others plain xor reductions.  Row c0 + 4r + g ends up in lane 8g + m(r).
-template <int KSTEPS, int R, bool FEW>
+template <int KSTEPS, int R, Load LOAD, class Ahead>
 __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint32_t d,
                                             const Query<KSTEPS>& q, const uint32_t* list,
-                                            uint32_t c0, uint32_t last) {
+                                            uint32_t c0, uint32_t last, Ahead ahead) {
   const uint32_t lane = lane_id(), g = lane >> 3, m = lane & 7u;
   const float* row[R];
 #pragma unroll
@@ -131,9 +168,7 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
   for (int r = 0; r < R; r++)
 #pragma unroll
     for (int i = 0; i < 4; i++) p[r][i] = 0.0f;
-  // steps whose loads are in flight together: all of them, but half of a long row's when many warps
-  // share the registers
-  constexpr int KB = KSTEPS > 8 && !FEW ? 8 : KSTEPS;
+  constexpr int KB = load_steps(KSTEPS, LOAD);
 #pragma unroll
   for (int k0 = 0; k0 < KSTEPS; k0 += KB) {
     float4 x[R][KB];
@@ -144,6 +179,7 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
         x[r][k] = 32u * (k0 + k) + 4u * m < d
                       ? __ldg(reinterpret_cast<const float4*>(row[r] + 32 * (k0 + k)))
                       : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k0 == 0) ahead();
 #pragma unroll
     for (int k = 0; k < KB && k0 + k < KSTEPS; k++) {
       if (32u * (k0 + k) + 4u * m < d) {
@@ -200,14 +236,8 @@ __device__ __forceinline__ float score_rows(const float* __restrict__ base, uint
   return (v[0] + v[2]) + (v[1] + v[3]);
 }
 
-// The lines of a row to L2, without waiting for them.
-__device__ __forceinline__ void prefetch_row(const float* row, uint32_t d) {
-  for (uint32_t c = 0; c < d; c += 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + c));
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(row + d - 1));  // a row that starts inside a line
-}
-
 // Distances of the lanes whose `newc` is set (FLT_MAX elsewhere), up to ROWS rows per pass.
-template <int KSTEPS, int ROWS, bool FEW>
+template <int KSTEPS, int ROWS, Load LOAD>
 __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTEPS>& q,
                                            uint32_t node, bool newc, uint32_t* list) {
   const uint32_t lane = lane_id();
@@ -215,24 +245,34 @@ __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTE
   const uint32_t nnew = __popc(newmask);
   const uint32_t ci = __popc(newmask & ((1u << lane) - 1u));
   if (newc) list[ci] = node;
-  if constexpr (FEW && KSTEPS > 8) {  // the rows of the later passes, which wait for each other
-    if (a.prefetch && newc && ci >= ROWS)
-      prefetch_row(a.base + static_cast<uint64_t>(node) * a.d, a.d);
-  }
   __syncwarp();
   float result = FLT_MAX;
   for (uint32_t c0 = 0; c0 < nnew; c0 += ROWS) {
     const uint32_t left = nnew - c0;
+    // The rows of the next pass to L2 while this one's are on their way.  The branch also keeps the
+    // compiler from moving loads between the FMAs, to save registers that these kernels have: without it
+    // 2432 queries x 512, Km = 32, took 745 instead of 334 us.
+    auto ahead = [&]() {
+      if constexpr (LOAD != Load::kMany && KSTEPS > 8) {
+        constexpr uint32_t T = 32 / ROWS;  // lanes per row
+        const uint32_t c = c0 + ROWS + lane / T;
+        if (a.prefetch && c < nnew) {
+          const float* row = a.base + static_cast<uint64_t>(list[c]) * a.d;
+          for (uint32_t i = 32u * (lane % T); i < a.d; i += 32u * T) prefetch_l2(row + i);
+          if (lane % T == T - 1) prefetch_l2(row + a.d - 1);  // a row that starts inside a line
+        }
+      }
+    };
     const uint32_t lc = ci - c0, r = lc >> 2;
     float total = 0.0f;
     uint32_t src = (lc & 3u) << 3;
     if (ROWS == 4 || left <= 4) {
-      total = score_rows<KSTEPS, 1, FEW>(a.base, a.d, q, list, c0, nnew - 1);
+      total = score_rows<KSTEPS, 1, LOAD>(a.base, a.d, q, list, c0, nnew - 1, ahead);
     } else if (ROWS <= 8 || left <= 8) {
-      total = score_rows<KSTEPS, 2, FEW>(a.base, a.d, q, list, c0, nnew - 1);
+      total = score_rows<KSTEPS, 2, LOAD>(a.base, a.d, q, list, c0, nnew - 1, ahead);
       src |= (r & 1u) << 2;
     } else if constexpr (ROWS == 16) {
-      total = score_rows<KSTEPS, 4, FEW>(a.base, a.d, q, list, c0, nnew - 1);
+      total = score_rows<KSTEPS, 4, LOAD>(a.base, a.d, q, list, c0, nnew - 1, ahead);
       src |= ((r >> 1) & 1u) << 2 | (r & 1u) << 1;
     }
     const float dd = __shfl_sync(kFull, total, src & 31u);
@@ -244,28 +284,10 @@ __device__ __forceinline__ float score_new(const SearchArgs& a, const Query<KSTE
 
 }  // namespace
 
-// Shape by measurement.  Rows per pass: eight short rows (up to 256 floats) whole in flight, four
-// long ones with half of each in flight, or four where eight would spill (short rows past 224
-// floats, Km > 32: 3745 -> 2711 us for 39k queries, Km = 64).  Long rows, eight at a time with a
-// quarter in flight: 4864 queries x 512, Km = 64: 1518 -> 1054 us, and 300k x 512 builds' searches
-// 19.7 + 30.9 -> 16.9 + 27.7 ms.  FEW, for calls with too few queries to fill the SMs, takes the
-// registers that hold 16 short or 8 long rows whole in flight: such a call lasts as long as its
-// longest chain of row reads (608 queries x 512, Km = 64: 601 -> 411 us).
-constexpr int search_rows(int km_s, int ksteps, bool few) {
-  if (few) return ksteps > 8 ? 8 : 16;
-  return ksteps > 8 || (ksteps == 8 && km_s > 1) ? 4 : 8;
-}
-
-// Warps per SM that the registers are allocated for: the fastest of 16..32.  One more or less costs
-// 1-3%, 16 or 32 cost 10-30% (too few warps, or spills).
-constexpr int search_warps(int km_s, int ksteps, bool few) {
-  return few ? 8 : ksteps > 8 ? 24 : km_s == 1 ? 23 : ksteps == 8 ? 20 : 21;
-}
-
-template <int KM_S, int KSTEPS, bool FEW>
+template <int KM_S, int KSTEPS, Load LOAD>
 __device__ __forceinline__ void search_queries(const SearchArgs& a) {
   constexpr uint32_t KM = 32u * KM_S;
-  constexpr int ROWS = search_rows(KM_S, KSTEPS, FEW);
+  constexpr int ROWS = search_rows(KM_S, KSTEPS, LOAD);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const uint32_t lane = lane_id();
   uint2* merged = reinterpret_cast<uint2*>(smem_raw);                // KM (key, id)
@@ -310,7 +332,7 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
       if (a.place) cand_id = a.place[cand_id];
       // scored for every query at once by k_seed_dists, or here
       const float dist = a.seed_dist ? a.seed_dist[static_cast<uint64_t>(qid) * 32u + lane]
-                                     : score_new<KSTEPS, ROWS, FEW>(a, q, cand_id, true, list);
+                                     : score_new<KSTEPS, ROWS, LOAD>(a, q, cand_id, true, list);
       cand_key = order_key(dist);
       ev += (lane == 0) ? 32u : 0u;
     }
@@ -367,7 +389,7 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
       const unsigned same = __match_any_sync(kFull, node);
       newc = node != kTomb && (same & lt_mask) == 0 && hash_test_and_set(hash, hmask, node);
       __syncwarp();
-      const float dist = score_new<KSTEPS, ROWS, FEW>(a, q, node, newc, list);
+      const float dist = score_new<KSTEPS, ROWS, LOAD>(a, q, node, newc, list);
       const unsigned scored = __ballot_sync(kFull, newc);
       ev += (lane == 0) ? __popc(scored) : 0u;
 #pragma unroll
@@ -471,15 +493,15 @@ __device__ __forceinline__ void search_queries(const SearchArgs& a) {
   }
 }
 
-template <int KSTEPS, bool FEW>
-__global__ void __launch_bounds__(32, search_warps(1, KSTEPS, FEW)) k_search_m32(SearchArgs a) {
-  search_queries<1, KSTEPS, FEW>(a);
+template <int KSTEPS, Load LOAD>
+__global__ void __launch_bounds__(32, search_warps(1, KSTEPS, LOAD)) k_search_m32(SearchArgs a) {
+  search_queries<1, KSTEPS, LOAD>(a);
 }
 
 // Km = 64, 96
-template <int KM_S, int KSTEPS, bool FEW>
-__global__ void __launch_bounds__(32, search_warps(KM_S, KSTEPS, FEW)) k_search_mk(SearchArgs a) {
-  search_queries<KM_S, KSTEPS, FEW>(a);
+template <int KM_S, int KSTEPS, Load LOAD>
+__global__ void __launch_bounds__(32, search_warps(KM_S, KSTEPS, LOAD)) k_search_mk(SearchArgs a) {
+  search_queries<KM_S, KSTEPS, LOAD>(a);
 }
 
 // Per warp: the merge buffer, the list of new candidates, the visited set and, for long rows, the
@@ -489,16 +511,16 @@ size_t search_smem(uint32_t km, uint32_t hash_slots, int ksteps, bool qshared) {
          (qshared ? static_cast<size_t>((ksteps + 3) / 4 * 4) * 128 : 0);
 }
 
-template <int KM_S, int KS, bool FEW>
+template <int KM_S, int KS, Load LOAD>
 static cudaError_t launch_search_k(const SearchArgs& a, int num_sms, size_t smem_optin,
                                    cudaStream_t st) {
   const size_t smem = search_smem(32u * KM_S, a.hash_slots, KS, kQueryShared<KS>);
   if (smem > smem_optin) return cudaErrorInvalidValue;
   void (*kern)(SearchArgs);
   if constexpr (KM_S == 1)
-    kern = k_search_m32<KS, FEW>;
+    kern = k_search_m32<KS, LOAD>;
   else
-    kern = k_search_mk<KM_S, KS, FEW>;
+    kern = k_search_mk<KM_S, KS, LOAD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
@@ -773,40 +795,52 @@ bool search_supported(uint32_t d, uint32_t km, uint32_t kp, uint32_t kd) {
 }
 
 template <int KM_S, int KS>
-static cudaError_t launch_search_few(const SearchArgs& a, bool few, int num_sms,
-                                     size_t smem_optin, cudaStream_t st) {
-  return few ? launch_search_k<KM_S, KS, true>(a, num_sms, smem_optin, st)
-             : launch_search_k<KM_S, KS, false>(a, num_sms, smem_optin, st);
+static cudaError_t launch_search_load(const SearchArgs& a, Load load, int num_sms,
+                                      size_t smem_optin, cudaStream_t st) {
+  if (load == Load::kFew) return launch_search_k<KM_S, KS, Load::kFew>(a, num_sms, smem_optin, st);
+  if constexpr (KS > 8)
+    if (load == Load::kMidLong)
+      return launch_search_k<KM_S, KS, Load::kMidLong>(a, num_sms, smem_optin, st);
+  if (load != Load::kMany) return launch_search_k<KM_S, KS, Load::kMid>(a, num_sms, smem_optin, st);
+  return launch_search_k<KM_S, KS, Load::kMany>(a, num_sms, smem_optin, st);
 }
 
 template <int KM_S>
-static cudaError_t launch_search_d(const SearchArgs& a, bool few, int num_sms, size_t smem_optin,
+static cudaError_t launch_search_d(const SearchArgs& a, Load load, int num_sms, size_t smem_optin,
                                    cudaStream_t st) {
-  if (a.d <= 224) return launch_search_few<KM_S, 7>(a, few, num_sms, smem_optin, st);
-  if (a.d <= 256) return launch_search_few<KM_S, 8>(a, few, num_sms, smem_optin, st);
-  return launch_search_few<KM_S, 16>(a, few, num_sms, smem_optin, st);
+  if (a.d <= 224) return launch_search_load<KM_S, 7>(a, load, num_sms, smem_optin, st);
+  if (a.d <= 256) return launch_search_load<KM_S, 8>(a, load, num_sms, smem_optin, st);
+  return launch_search_load<KM_S, 16>(a, load, num_sms, smem_optin, st);
 }
 
 cudaError_t launch_search(const SearchArgs& a, int num_sms, size_t smem_optin, cudaStream_t st) {
   if (!search_supported(a.d, a.km, a.kp, a.kd)) return cudaErrorInvalidValue;
   if (a.rows != 0 && a.rows != 8 && a.rows != 16) return cudaErrorInvalidValue;
-  // Few queries: up to eight per SM, one resident round of the FEW kernels.  At sixteen per SM the
-  // others are as fast for long rows and faster for short ones (2432 queries x 200, Km = 32: 136
-  // against 152 us; 1216: 125 against 103).
-  const uint64_t nq = a.queries ? a.nq : a.n;
-  const bool few = nq <= static_cast<uint64_t>(num_sms) * 8 || (a.rows == 16 && a.km == 32);
+  // The kernels that hold all the queries in one resident round, up to 16 per SM: a second round of few
+  // queries lasts as long as the first.  Queries never asked before, by class (kFew, kMidLong, kMid,
+  // kMany; us):
+  //   1000 x 200, Km = 32:  119,   -, 125, 162      2432 x 200, Km = 32:  160,   -, 124, 149
+  //   1300 x 512, Km = 32:  312, 312, 347, 469      2432 x 512, Km = 32:  376, 335, 358, 473
+  //   1300 x 384, Km = 96:    -, 556, 559, 650      2432 x 384, Km = 96:    -, 737, 608, 694
+  // Rows of up to 64 floats leave the registers of kMid unused (1300 x 64: 129, 124).  Past 16 per SM
+  // kMany is faster on most graphs (3000 x 320, Km = 32: 309, 288; 400k points, 3000 x 512: 212, 185) but
+  // not on all (200k points with one long chain, 3000 x 512: 360, 481).
+  const uint64_t nq = a.queries ? a.nq : a.n, sms = static_cast<uint64_t>(num_sms);
+  const Load load = nq <= sms * 8 || (a.rows == 16 && a.km == 32) ? Load::kFew
+                    : nq > sms * 16 || a.d <= 64                 ? Load::kMany
+                    : nq <= sms * 12                             ? Load::kMidLong
+                                                                 : Load::kMid;
   // Few long rows: the passes of an iteration wait for each other, so rows that lie in DRAM (queries
-  // not asked before) cost one DRAM latency per pass.  Sending the later passes' rows to L2 first pays
-  // there and costs a little on rows already in L2.  16 queries x 512, Km = 32, L2 flushed 224 -> 209
-  // us, asked again 183 -> 184; 16 x 384, Km = 96, 495 -> 449 and 296 -> 308.  Up to 320 floats it
-  // cost as much as it gave (260: 139 -> 132 and 110 -> 113), and with more than two queries per SM
-  // other queries hide the latency (1000 x 512: 300 -> 302 and, 400k points, 125 -> 134).
+  // not asked before) cost one DRAM latency per pass unless they are sent to L2 a pass ahead.  Km = 32,
+  // new queries and the same again: 16 x 512 297 -> 277 and 232 -> 231 us, 300 x 384 228 -> 224 and 186
+  // -> 194.  Up to 320 floats it cost as much as it gave, and with more than two queries per SM other
+  // queries hide the latency.
   SearchArgs b = a;
-  b.prefetch = a.d > 320 && nq <= static_cast<uint64_t>(num_sms) * 2;
+  b.prefetch = a.d > 320 && nq <= sms * 2;
   switch (a.km / 32) {
-    case 1: return launch_search_d<1>(b, few, num_sms, smem_optin, st);
-    case 2: return launch_search_d<2>(b, few, num_sms, smem_optin, st);
-    default: return launch_search_d<3>(b, few, num_sms, smem_optin, st);
+    case 1: return launch_search_d<1>(b, load, num_sms, smem_optin, st);
+    case 2: return launch_search_d<2>(b, load, num_sms, smem_optin, st);
+    default: return launch_search_d<3>(b, load, num_sms, smem_optin, st);
   }
 }
 

@@ -888,7 +888,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     bool ok = true;
     uint32_t t = 0;
     const uint32_t chunks = n_tiles * kCpt;  // this thread's 32-column chunks per M tile
-    for (uint32_t st = blockIdx.x; ok && st < q_tiles; st += gridDim.x) {
+    uint32_t st = blockIdx.x;
+    for (; st < q_tiles; st += gridDim.x) {
       if (!swept(st)) continue;
       uint32_t qrow[MT], cnt[MT];
       bool valid[MT];
@@ -988,7 +989,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-      if (MODE == kFilter && ok) {
+      if (!ok) break;
+      if (MODE == kFilter) {
         // each half of a row keeps its candidates in its own half of the row's list
 #pragma unroll
         for (uint32_t m = 0; m < MT; m++)
@@ -998,9 +1000,19 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
       }
     }
-    if (!ok && lane == 0) {
-      raise_error(a.status, kErrWait);
-      *stop = 1;
+    if (!ok) {
+      if (lane == 0) {
+        raise_error(a.status, kErrWait);
+        *stop = 1;
+      }
+      // the queries not reached have no candidates: the kernels that follow read rows by id
+      if (MODE == kFilter)
+        for (; st < q_tiles; st += gridDim.x)
+#pragma unroll
+          for (uint32_t m = 0; m < MT; m++) {
+            const uint32_t r = st * rows_per_tile + m * kRows + row;
+            if (r < a.nq) a.cand_cnt[static_cast<uint64_t>(r) * 2 + half] = 0;
+          }
     }
   }
   fence_before();

@@ -403,7 +403,8 @@ __global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneA
   };
   fetch(blockIdx.x);
 
-  for (uint64_t t = blockIdx.x; t < sh.tiles; t += gridDim.x, it++) {
+  uint64_t t = blockIdx.x;
+  for (; t < sh.tiles; t += gridDim.x, it++) {
     const uint64_t b = t * P + node;
     const bool bval = b < a.n;
     uint32_t x = x_next;
@@ -581,6 +582,10 @@ __global__ void __launch_bounds__(kTile, S <= 3 ? 4 : 3) k_prune_tc(const PruneA
     }
     fence_before();  // the TMEM reads above precede the next tile's first MMA
   }
+  // After a wait that gave up, the nodes not reached keep nothing: the kernels that follow read counts.
+  if (!ok)
+    for (; t < sh.tiles; t += gridDim.x)
+      if (slot == 0 && t * P + node < a.n) a.pruned_num[t * P + node] = 0;
   cp_wait<0>();  // no copy lands after the CTA exits
   if (lane == 0) {
     if (ev) atomicAdd(a.evals, static_cast<unsigned long long>(ev));

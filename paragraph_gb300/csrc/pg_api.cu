@@ -178,10 +178,11 @@ void release_ws(pg_handle h) {
   h->ws_bytes = 0;
 }
 
-// Whether a workspace of this size is there or could be allocated now.  Asked before a build gives up
-// the workspace it has for a larger one that it can do without.
+// Whether a workspace of this size is there or worth trying for.  A build asks before it gives up the
+// workspace it has for a larger one that it can do without; with none to lose it just tries (asking
+// takes 20 us).
 bool room_for_ws(pg_handle h, size_t bytes) {
-  if (bytes <= h->ws_bytes) return true;
+  if (bytes <= h->ws_bytes || !h->ws) return true;
   size_t avail = 0, all = 0;
   if (cudaMemGetInfo(&avail, &all) != cudaSuccess) {
     cudaGetLastError();

@@ -72,18 +72,6 @@ __global__ void k_match_rows(const uint32_t* __restrict__ gt, uint32_t gt_k, uin
   }
 }
 
-__global__ void k_validate_ids(const uint32_t* __restrict__ ids, uint64_t count, uint64_t n,
-                               uint32_t* status) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  bool bad = false;
-  for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < count;
-       i += stride) {
-    const uint32_t v = ids[i];
-    bad |= (v != kTomb && v >= n);
-  }
-  if (__any_sync(kFull, bad) && lane_id() == 0) raise_error(status, kErrBadId);
-}
-
 // ------------------------------------------------------------------ one node's list
 // Lists of up to CAP = 32 W entries and the team of W warps that works on one: thread t holds
 // entry t while it is gathered and sorted.
@@ -916,12 +904,6 @@ cudaError_t launch_match_rows(const uint32_t* gt, uint32_t gt_k, uint64_t n,
                               const uint32_t* winner, uint32_t* out, int num_sms,
                               cudaStream_t st) {
   k_match_rows<<<grid_for(n * gt_k, 256, num_sms, 8), 256, 0, st>>>(gt, gt_k, n, winner, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_validate_ids(const uint32_t* ids, uint64_t count, uint64_t n,
-                                uint32_t* status, int num_sms, cudaStream_t st) {
-  k_validate_ids<<<grid_for(count, 256, num_sms, 8), 256, 0, st>>>(ids, count, n, status);
   return cudaGetLastError();
 }
 

@@ -205,8 +205,6 @@ cudaError_t launch_restore(const uint32_t* rows, uint64_t n, uint32_t deg, const
 cudaError_t launch_match_rows(const uint32_t* gt, uint32_t gt_k, uint64_t n,
                               const uint32_t* winner, uint32_t* out, int num_sms,
                               cudaStream_t st);
-cudaError_t launch_validate_ids(const uint32_t* ids, uint64_t count, uint64_t n,
-                                uint32_t* status, int num_sms, cudaStream_t st, float* diag = nullptr);
 cudaError_t launch_prune_reverse(const PruneArgs& a, bool phase1, int num_sms, cudaStream_t st);
 // Reverse edges as CSR over n destinations: offs = exclusive scan of indeg, edges grouped by
 // destination holding the source row index.  `rows` pruned rows are scanned (0 = n).

@@ -30,10 +30,10 @@ __device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
 }
 
 // Rows of at least this many floats (1 KB) are read with 256-bit loads by the exact chains of the
-// prunes and the merges when 32-byte aligned (their launchers pick the WIDE kernels): such
-// rows mostly come from DRAM, where half the load requests pay (measured at 1M x 512: merges
-// 251 -> 190 ms per build); the shorter rows of the L2-resident 1M x 200 workload were measured
-// faster with the float4 kernels.
+// prunes and the merges when 32-byte aligned (their launchers pick the WIDE kernels): half the load
+// requests of float4.  Builds without screening: 120k x 512 31.5 -> 28.0 ms, 300k x 512 70.8 -> 62.4,
+// 120k x 256 12.1 -> 10.8; with it about 1%.  The line is older than the kernels: rows of 200 floats
+// would gain too (120k 8.6 -> 8.1 ms without screening, nothing with it).
 constexpr uint32_t kWideRowFloats = 256;
 
 // One FMA chain over d = 0..D-1: distance_between (Gbuilder.cuh:785-797), -(sum x[d]*y[d]).

@@ -5,7 +5,8 @@
 //   winner    n u32                   projection winner key per base (K0)
 //   pruned    n x P u32 + n counts    RNG-pruned out-lists (K2)
 //   indeg     n u32 -> offs n+1       reverse-edge counts -> CSR offsets
-//   edges     sum(pruned counts) u32  reverse sources grouped by destination (CSR)
+//   edges     sum(pruned counts) u32  reverse sources grouped by destination (CSR); 8 bytes each in
+//                                     builds, with the edge's distance
 //   reverse   n x R u32 + n counts    first R sources per destination, ascending (K2's add_reverse)
 //   graph     n x degree u32          merged + pruned out-lists, tomb padded (K3)
 // A team of warps sized to the list owns one node in K2 and K3, one thread per candidate; a warp

@@ -63,14 +63,15 @@ __device__ __forceinline__ void hash_clear(uint32_t* t, uint32_t slots) {
 
 // ---------------------------------------------------------------------------------------------
 // What bounds the search: issue slots and the latency of each iteration's chain (list -> graph row
-// -> visited set -> candidate rows -> merge), with L2 (D = 200) or DRAM (D = 512 at a million
-// points) behind the row loads.  Hence few instructions per iteration and many resident warps:
+// -> visited set -> candidate rows -> merge), with L2 behind the row loads (DRAM where a large base is
+// not relocated, and for queries not asked before).  Hence few instructions per iteration and many
+// resident warps:
 //   * rows come by plain coalesced loads.  One cp.async.bulk per row into shared memory (the
 //     earlier scheme) is issued lane by lane and held 6-16 KB of shared memory per warp;
 //   * 32-bit keys, one pass over the entering candidates only, and the same ranks for the output
 //     instead of two 64-element sorting networks per query;
-//   * registers held to about 80 (20-24 warps per SM); for rows over 256 floats the query stays in
-//     shared memory.
+//   * registers held to about 80 (20-24 warps per SM) where there are queries for that many; for rows
+//     over 256 floats the query stays in shared memory.
 // Both rounds on the caller's rows, 1M x 200, Km = 32: 25.5 + 22.5 -> 18.2 + 15.1 ms; 400k x 512,
 // Km = 32: 6.6 + 10.6 -> 1.4 + 5.8 ms; 200k x 128, Km = 96: 16 + 12.6 -> 10.2 + 7.8 ms; 300k x 512,
 // Km = 64: 38 + 59.4 -> 23.3 + 58.5 ms (DRAM-bound; on relocated rows 16.9 + 27.7).
